@@ -31,6 +31,7 @@ const char *sched_name(Sched s) {
         case Sched::LANE_REDUCE: return "lane_reduce";
         case Sched::OUTER_REDUCE: return "outer_reduce";
         case Sched::SCAN1D: return "scan1d";
+        case Sched::AXIS_SCAN: return "axis_scan";
         case Sched::SERIAL: return "serial";
         case Sched::TILE2D: return "tile2d";
     }
@@ -53,7 +54,8 @@ int64_t LaunchUnit::work_items() const {
             return (rows * cols + per - 1) / per;
         }
         case Sched::OUTER_REDUCE: return (rows * cols + kThreads - 1) / kThreads;
-        case Sched::SCAN1D: return chunks;  // chunks: work items of the phase
+        case Sched::SCAN1D:
+        case Sched::AXIS_SCAN: return chunks;  // chunks: work items of the phase
         case Sched::SERIAL: return 1;
         case Sched::TILE2D: return (rows + V - 1) / V * ((cols + 63) / 64);  // V: rows per tile
     }
@@ -161,6 +163,11 @@ template <typename T> __device__ __forceinline__ T bh_shfl_xor(T v, int m) {
 }
 
 template <typename T> __device__ __forceinline__ T bh_shfl_idx(T v, int src) {
+    if (sizeof(T) <= 4) {
+        int x = 0; memcpy(&x, &v, sizeof(T));
+        x = __shfl_sync(0xffffffffu, x, src);
+        T r; memcpy(&r, &x, sizeof(T)); return r;
+    }
     long long x[2] = {0, 0};
     memcpy(x, &v, sizeof(T));
     x[0] = __shfl_sync(0xffffffffu, x[0], src);
@@ -169,6 +176,11 @@ template <typename T> __device__ __forceinline__ T bh_shfl_idx(T v, int src) {
 }
 
 template <typename T> __device__ __forceinline__ T bh_shfl_up(T v, int d) {
+    if (sizeof(T) <= 4) {
+        int x = 0; memcpy(&x, &v, sizeof(T));
+        x = __shfl_up_sync(0xffffffffu, x, d);
+        T r; memcpy(&r, &x, sizeof(T)); return r;
+    }
     long long x[2] = {0, 0};
     memcpy(x, &v, sizeof(T));
     x[0] = __shfl_up_sync(0xffffffffu, x[0], d);
@@ -3988,6 +4000,366 @@ __device__ __forceinline__ bool bh_await(const unsigned *flag, const unsigned *a
     return u;
 }
 
+// ---------------------------------------------------------------------------------- AXIS_SCAN
+// An accumulate along one axis of an array of two or more dimensions (P threaded ranks around one
+// innermost swept loop): the running value stays in a register and the swept axis is cut into
+// chunks where the points alone leave the GPU idle. With more than one chunk there are two units:
+// totals (each chunk folded) and the scan (each chunk starts from the fold, in chunk order, of the
+// totals before it, so the sum's order depends on the shapes only). FLAT, which ran these nests
+// before with one thread per point, re-read the value it had just stored for every element: the
+// summed-area table of a 4000x4099 float32 image (one scan along each axis) took 3.74 ms and takes
+// 82 us here; one read and one write of both scans are 41 us at the measured copy rate.
+//
+// Two layouts of the points on threads:
+//   columns  a thread per (point, chunk); neighbouring threads hold neighbouring points, so the
+//            loads of one element per thread are coalesced when the innermost threaded rank is
+//            contiguous. The axis is read twice when it is cut, the second time partly from L2: 28 us
+//            a unit at that size. kScanUnroll loads per thread in flight and about kAxisScanThreads
+//            threads (4 and 16 loads, 1024 and 2048 threads per SM measured 3 to 18 % slower; more
+//            chunks make the fold of the totals longer: half the chunks per thread on average).
+//   rows     for a contiguous swept axis of at least a warp's length: a warp per (point, chunk)
+//            walks it in strips of 32 elements, coalesced whatever the alignment, with a shuffle
+//            scan per strip (independent of the running value, so kScanUnroll strips overlap) and
+//            one addition per strip on the serial chain. 34 us for 131 MB at that size; bound by
+//            instruction issue (58 instructions per strip took 42 us; loading the next strips
+//            ahead gave nothing).
+constexpr int kScanUnroll = 8;
+constexpr int64_t kAxisScanThreads = 148 * 1536; // columns: (point, chunk) threads aimed at
+constexpr int64_t kAxisScanMinRows = 32;         // columns: shortest chunk
+constexpr int64_t kAxisScanWarps = 148 * 16;     // rows: (point, chunk) warps aimed at
+constexpr int64_t kAxisScanMinRun = 1024;        // rows: shortest chunk (elements)
+
+struct AxisScan {
+    const LoopB *sub = nullptr;     // the swept loop
+    InstrPtr acc;                   // its accumulate
+    vector<InstrPtr> before, after; // the elementwise instructions around it, in order
+    bool rows = false;              // layout
+    int64_t chunks = 1, chunk_len = 0;
+};
+
+// Whether the kernel's threaded nest with innermost threaded loop `inner` is an AXIS_SCAN: loops
+// that seed the accumulate's output (dropped: the scan starts from the identity), one innermost
+// loop with one accumulate among elementwise instructions, then elementwise loops of the same
+// length. Elements of one point are computed by different threads, and the totals unit computes
+// the instructions before the accumulate without storing them, so: every array the nest writes is
+// touched through one view only, and no instruction before the accumulate reads an array that one
+// of them (itself included) writes later. Floating-point products keep one running product per
+// point: a chunk's own product can overflow where the running one does not.
+bool axis_scan_applicable(const LoopB &inner, int64_t points, unsigned P, const CodegenOptions &opt, AxisScan &as) {
+    if (opt.bounds_check) return false;
+    for (const Block &b : inner._block_list) {
+        if (b.isInstr()) {
+            if (bh_opcode_is_system(b.getInstr()->opcode)) continue;
+            return false;
+        }
+        const LoopB &l = b.getLoop();
+        if (l.isSystemOnly()) continue;
+        if (!l.isInnermost()) return false;
+        if (!l._sweeps.empty()) {
+            if (as.sub != nullptr || l._sweeps.size() != 1) return false;
+            as.sub = &l;
+            as.acc = *l._sweeps.begin();
+        }
+    }
+    if (as.sub == nullptr) return false;
+    const InstrPtr &acc = as.acc;
+    if (acc->opcode != BH_ADD_ACCUMULATE && acc->opcode != BH_MULTIPLY_ACCUMULATE) return false;
+    const bh_view &out = acc->operand[0];
+    const bh_type t = out.base->dtype();
+    if (acc->opcode == BH_MULTIPLY_ACCUMULATE && !bh_type_is_integer(t)) return false;
+    if (t == bh_type::BOOL || acc->operand[1].isConstant() || acc->operand[1].base == out.base) return false;
+    if (out.ndim != static_cast<int64_t>(P) + 1 || acc->sweep_axis() != static_cast<int64_t>(P)) return false;
+    bool seen = false;
+    for (const Block &b : inner._block_list) {
+        if (b.isInstr()) continue;
+        const LoopB &l = b.getLoop();
+        if (l.isSystemOnly()) continue;
+        if (!seen && &l != as.sub) {
+            // before the scan: only the loop that seeds its output
+            const vector<InstrPtr> is = jitk::all_instr(l);
+            for (const InstrPtr &i : is) {
+                if (bh_opcode_is_system(i->opcode)) continue;
+                // the loop that seeds the output's first element along the axis
+                if (!(i->opcode == BH_IDENTITY && i->operand.size() == 2 && i->operand[1].isConstant() && l.size <= 1 &&
+                      i->operand[0].base == out.base && i->operand[0].start == out.start))
+                    return false;
+            }
+            continue;
+        }
+        if (l.size != as.sub->size) return false;
+        for (const Block &ib : l._block_list) {
+            const InstrPtr &i = ib.getInstr();
+            const bh_opcode op = i->opcode;
+            if (i == acc) {
+                seen = true;
+                continue;
+            }
+            if (bh_opcode_is_system(op)) continue;
+            if (bh_opcode_is_sweep(op) || op == BH_GATHER || op == BH_SCATTER || op == BH_COND_SCATTER || i->operand.empty())
+                return false;
+            (seen ? as.after : as.before).push_back(i);
+        }
+    }
+    map<const bh_base *, set<ViewKey>> touched;
+    set<const bh_base *> written, read_before;
+    auto touch = [&](const InstrPtr &i) {
+        for (const bh_view &v : i->operand)
+            if (!v.isConstant()) touched[v.base].insert(ViewKey(v));
+        written.insert(i->operand[0].base);
+    };
+    for (const InstrPtr &i : as.before) {
+        for (size_t o = 1; o < i->operand.size(); ++o)
+            if (!i->operand[o].isConstant() && !written.count(i->operand[o].base)) read_before.insert(i->operand[o].base);
+        if (read_before.count(i->operand[0].base)) return false;
+        touch(i);
+    }
+    touched[out.base].insert(ViewKey(out));
+    touched[acc->operand[1].base].insert(ViewKey(acc->operand[1]));
+    written.insert(out.base);
+    for (const InstrPtr &i : as.before)
+        for (const bh_view &v : i->operand)
+            if (!v.isConstant() && v.base == out.base) return false;
+    for (const InstrPtr &i : as.after) {
+        if (i->operand[0].base == out.base) return false;
+        touch(i);
+    }
+    for (const bh_base *b : written)
+        if (touched[b].size() != 1) return false;
+    // Layout: rows when every array walked along the axis has unit stride there.
+    const int64_t n = as.sub->size;
+    bool unit = n >= 32;
+    vector<InstrPtr> all = as.before;
+    all.insert(all.end(), as.after.begin(), as.after.end());
+    all.push_back(acc);
+    for (const InstrPtr &i : all)
+        for (const bh_view &v : i->operand)
+            if (!v.isConstant() && v.ndim == static_cast<int64_t>(P) + 1 && v.stride[P] != 1 && v.stride[P] != 0) unit = false;
+    as.rows = unit;
+    const int64_t want = as.rows ? kAxisScanWarps : kAxisScanThreads, least = as.rows ? kAxisScanMinRun : kAxisScanMinRows;
+    const int64_t unit_len = as.rows ? 32 * kScanUnroll : kScanUnroll;
+    const int64_t c = max<int64_t>(1, min((want + max<int64_t>(points, 1) - 1) / max<int64_t>(points, 1), n / least));
+    as.chunk_len = max(unit_len, ((n + c - 1) / c + unit_len - 1) / unit_len * unit_len);
+    as.chunks = max<int64_t>(1, (n + as.chunk_len - 1) / as.chunk_len);
+    return true;
+}
+
+vector<LaunchUnit> lower_axis_scan(const LoopB &loop, unsigned P, const CodegenOptions &opt) {
+    const Block holder(loop);
+    const LoopB &L = holder.getLoop();
+    const vector<const LoopB *> chain = jitk::get_first_loop_blocks(L);
+    int64_t points = 1;
+    for (unsigned r = 0; r < P; ++r) points *= chain[r]->size;
+    AxisScan as;
+    if (!axis_scan_applicable(*chain[P - 1], points, P, opt, as)) throw runtime_error("lower_axis_scan(): not a scan");
+    const InstrPtr &acc = as.acc;
+    const bh_view &outv = acc->operand[0];
+    const bh_type t = outv.base->dtype();
+    const string T = cuda_type(t);
+    const bh_opcode rop = scan_reduce_op(acc->opcode);
+    const string ident = constant_literal(jitk::sweep_identity(rop, t));
+    const string ix = "i" + to_string(P);
+    vector<LaunchUnit> units;
+    for (int phase = as.chunks > 1 ? 0 : 1; phase < 2; ++phase) {
+        const bool scan = phase == 1;
+        LaunchUnit u;
+        u.sched = Sched::AXIS_SCAN;
+        u.rows = points;
+        u.cols = as.sub->size;
+        Symbols sym = build_symbols({&holder}, {});
+        ParamLayout pl;
+        add_common_fields(sym, pl, opt);
+        pl.add(work_field(points), "bh_i64", "points");
+        pl.add(work_field(as.chunks), "bh_i64", "chunks");
+        pl.add(work_field(as.chunk_len), "bh_i64", "chunk_len");
+        u.chunks = as.rows ? (points * as.chunks + kThreads / 32 - 1) / (kThreads / 32)
+                           : (points + kThreads - 1) / kThreads * as.chunks;
+        pl.add(work_field(u.chunks), "bh_i64", "work");
+        ParamField fs{ParamField::SCRATCH};
+        pl.add(fs, "unsigned char*", "scratch");
+        const string n = "(bh_i64)p.n" + to_string(sym.loop_id.at(as.sub));
+        // Inputs that are only read are loaded kScanUnroll elements ahead of the instructions.
+        vector<bh_view> pre = preloadable_views(*as.sub, L, sym);
+        set<const bh_base *> written;
+        for (const InstrPtr &i : jitk::all_instr(L))
+            if (!i->operand.empty() && !i->operand[0].isConstant()) written.insert(i->operand[0].base);
+        const bh_view &inv = acc->operand[1];
+        if (!sym.temps.count(inv.base) && !written.count(inv.base) &&
+            find_if(pre.begin(), pre.end(), [&](const bh_view &v) { return v == inv; }) == pre.end())
+            pre.push_back(inv);
+
+        stringstream body;
+        Emitter em(sym, body, opt);
+        body << "__device__ __forceinline__ void bh_work(const P &p, bh_i64 w) {\n";
+        body << pointer_locals(sym);
+        body << "    " << T << "* totals = (" << T << "*)p.scratch;\n";
+        if (as.rows) {
+            body << "    const int lane = threadIdx.x & 31;\n";
+            body << "    const bh_i64 item = w * " << kThreads / 32 << " + (threadIdx.x >> 5);\n";
+            body << "    if (item >= p.points * p.chunks) return;\n"; // the whole warp
+            body << "    const bh_i64 pt = item / p.chunks, chunk = item - pt * p.chunks;\n";
+        } else {
+            body << "    const bh_i64 pb = w / p.chunks, chunk = w - pb * p.chunks;\n";
+            body << "    const bh_i64 pt = pb * " << kThreads << " + threadIdx.x;\n";
+            body << "    if (pt >= p.points) return;\n";
+        }
+        body << "    bh_i64 rem = pt;\n";
+        for (int r = static_cast<int>(P) - 1; r >= 0; --r) {
+            const int lid = sym.loop_id.at(chain[static_cast<size_t>(r)]);
+            if (r == 0) {
+                body << "    const bh_i64 i0 = rem;\n";
+            } else {
+                body << "    const bh_i64 i" << r << " = rem % p.n" << lid << "; rem /= p.n" << lid << ";\n";
+            }
+        }
+        body << "    (void)rem;\n";
+        body << "    const bh_i64 lo = chunk * p.chunk_len;\n";
+        body << "    const bh_i64 hi = min(lo + p.chunk_len, " << n << ");\n";
+        body << "    " << T << " run = " << ident << ";\n";
+        if (scan && as.chunks > 1) {
+            // The value the chunk starts from: the totals of the chunks before it, in order.
+            if (as.rows) {
+                body << "    for (bh_i64 b = 0; b < chunk; b += 32) {\n";
+                body << "        " << T << " x = " << ident << ";\n";
+                body << "        if (b + lane < chunk) x = bh_ldcg(totals + pt * p.chunks + b + lane);\n";
+                body << "#pragma unroll\n";
+                body << "        for (int d = 1; d < 32; d <<= 1) {\n";
+                body << "            const " << T << " y = bh_shfl_up(x, d);\n";
+                body << "            if (lane >= d) x = " << reduce_expr(rop, "y", "x") << ";\n";
+                body << "        }\n";
+                body << "        const " << T << " s = bh_shfl_idx(x, 31);\n";
+                body << "        run = " << reduce_expr(rop, "run", "s") << ";\n";
+                body << "    }\n";
+            } else {
+                body << "    {\n";
+                body << "        bh_i64 c = 0;\n";
+                body << "        for (; c + 8 <= chunk; c += 8) {\n";
+                body << "            " << T << " x[8];\n";
+                body << "#pragma unroll\n";
+                body << "            for (int j = 0; j < 8; ++j) x[j] = bh_ldcg(totals + (c + j) * p.points + pt);\n";
+                body << "#pragma unroll\n";
+                body << "            for (int j = 0; j < 8; ++j) run = " << reduce_expr(rop, "run", "x[j]") << ";\n";
+                body << "        }\n";
+                body << "        for (; c < chunk; ++c) {\n";
+                body << "            const " << T << " x = bh_ldcg(totals + c * p.points + pt);\n";
+                body << "            run = " << reduce_expr(rop, "run", "x") << ";\n";
+                body << "        }\n";
+                body << "    }\n";
+            }
+        }
+        const int U = kScanUnroll;
+        const int step = as.rows ? 32 * U : U;
+        const string idx = "const bh_i64 " + ix + " = base + j" + (as.rows ? " * 32 + lane;" : ";");
+        hoist_views(em, *as.sub, static_cast<int>(P), body, 4);
+        for (const Block &b : chain[P - 1]->_block_list)
+            if (!b.isInstr() && &b.getLoop() != as.sub && b.getLoop()._sweeps.empty() && scan)
+                hoist_views(em, b.getLoop(), static_cast<int>(P), body, 4);
+        if (scan && !sym.temps.count(outv.base) && !em.hoisted.count(sym.view_id.at(outv))) {
+            const string nm = "hp" + to_string(em.hoisted.size());
+            body << "    " << T << "* __restrict__ " << nm << " = a" << sym.param_id.at(outv.base) << " + "
+                 << em.index_expr(outv, BH_MAXDIM, {-1, 0}, static_cast<int>(P)) << ";\n";
+            em.hoisted[sym.view_id.at(outv)] = nm;
+        }
+        body << "    for (bh_i64 base = lo; base < hi; base += " << step << ") {\n";
+        for (int path = 0; path < 2; ++path) {
+            // path 0: a full block of elements without bounds checks; path 1: the last block.
+            body << (path == 0 ? "        if (base + " + to_string(step) + " <= hi) {\n" : "        } else {\n");
+            const string guard = path == 0 ? "" : ix + " >= hi";
+            Scope scope;
+            declare_chain_temps(em, sym, scope, chain, P, body, 12);
+            emit_preload(em, pre, U, idx, guard, scope, body, 12);
+            const string sp(12, ' ');
+            // Values of the instructions before the accumulate: one register per element of the
+            // block (rows: the instructions after it run after the strip scans).
+            set<const bh_base *> local;
+            for (const vector<InstrPtr> *is : {&as.before, &as.after})
+                for (const InstrPtr &i : *is)
+                    for (const bh_view &v : i->operand)
+                        if (!v.isConstant() && sym.temps.count(v.base) && !scope.is_tmp(v.base)) local.insert(v.base);
+            if (sym.temps.count(inv.base) && !scope.is_tmp(inv.base)) local.insert(inv.base);
+            if (!scan)
+                for (const InstrPtr &i : as.before)
+                    if (!scope.is_tmp(i->operand[0].base)) local.insert(i->operand[0].base);
+            vector<const bh_base *> ordered(local.begin(), local.end());
+            sort(ordered.begin(), ordered.end(),
+                 [&](const bh_base *a, const bh_base *b) { return sym.base_id.at(a) < sym.base_id.at(b); });
+            for (const bh_base *b : ordered)
+                body << sp << cuda_type(b->dtype()) << " q" << sym.base_id.at(b) << "[" << U << "];\n";
+            for (const vector<InstrPtr> *is : {&as.before, &as.after})
+                for (const InstrPtr &i : *is)
+                    for (const bh_view &v : i->operand)
+                        if (!v.isConstant() && local.count(v.base))
+                            scope.repl[ViewKey(v)] = "q" + to_string(sym.base_id.at(v.base)) + "[j]";
+            if (local.count(inv.base)) scope.repl[ViewKey(inv)] = "q" + to_string(sym.base_id.at(inv.base)) + "[j]";
+            auto emit_after = [&](int ind, const string &value) {
+                const string s2(static_cast<size_t>(ind), ' ');
+                if (!sym.temps.count(outv.base)) body << s2 << em.array_ref(outv) << " = " << value << ";\n";
+                const auto saved = scope.repl;
+                scope.repl[ViewKey(outv)] = value;
+                for (const InstrPtr &i : as.after) em.write_instr(*i, scope, ind);
+                scope.repl = saved;
+            };
+            if (as.rows) {
+                body << sp << T << " xs[" << U << "];\n";
+                body << "#pragma unroll\n";
+                body << sp << "for (int j = 0; j < " << U << "; ++j) {\n";
+                body << sp << "    xs[j] = " << ident << ";\n";
+                body << sp << "    " << idx << "\n";
+                body << sp << "    " << (path == 0 ? "" : "if (" + ix + " < hi) ") << "{\n";
+                for (const InstrPtr &i : as.before) em.write_instr(*i, scope, 20);
+                body << sp << "        xs[j] = " << em.name(inv, scope) << ";\n";
+                body << sp << "    }\n" << sp << "}\n";
+                body << "#pragma unroll\n";
+                body << sp << "for (int d = 1; d < 32; d <<= 1) {\n";
+                body << "#pragma unroll\n";
+                body << sp << "    for (int j = 0; j < " << U << "; ++j) {\n";
+                body << sp << "        const " << T << " y = bh_shfl_up(xs[j], d);\n";
+                body << sp << "        if (lane >= d) xs[j] = " << reduce_expr(rop, "y", "xs[j]") << ";\n";
+                body << sp << "    }\n" << sp << "}\n";
+                body << "#pragma unroll\n";
+                body << sp << "for (int j = 0; j < " << U << "; ++j) {\n";
+                body << sp << "    const " << T << " s = bh_shfl_idx(xs[j], 31);\n";
+                if (scan) {
+                    body << sp << "    " << idx << "\n";
+                    body << sp << "    " << (path == 0 ? "" : "if (" + ix + " < hi) ") << "{\n";
+                    body << sp << "        const " << T << " val = " << reduce_expr(rop, "run", "xs[j]") << ";\n";
+                    emit_after(20, "val");
+                    body << sp << "    }\n";
+                }
+                body << sp << "    run = " << reduce_expr(rop, "run", "s") << ";\n";
+                body << sp << "}\n";
+            } else {
+                if (path == 0) body << "#pragma unroll\n";
+                body << sp << "for (int j = 0; j < " << U << "; ++j) {\n";
+                body << sp << "    " << idx << "\n";
+                if (path == 1) body << sp << "    if (" << guard << ") break;\n";
+                for (const InstrPtr &i : as.before) em.write_instr(*i, scope, 16);
+                body << sp << "    run = " << reduce_expr(rop, "run", em.name(inv, scope)) << ";\n";
+                if (scan) emit_after(16, "run");
+                body << sp << "}\n";
+            }
+        }
+        body << "        }\n    }\n";
+        if (!scan) {
+            if (as.rows) {
+                body << "    if (lane == 0) totals[pt * p.chunks + chunk] = run;\n";
+            } else {
+                body << "    totals[chunk * p.points + pt] = run;\n";
+            }
+        }
+        body << "}\n" << kWrappers;
+        u.fields = pl.fields;
+        u.scan_bytes = as.chunks > 1 ? points * as.chunks * static_cast<int64_t>(bh_type_size(t)) : 0;
+        u.algorithmic_bytes = scan ? unit_bytes(sym, vector<const Block *>{&holder}) : 0;
+        u.elements = points * as.sub->size;
+        if (scan && (as.rows || as.chunks > 1))
+            u.red_orders.emplace_back(acc->origin_id, string(as.rows ? "strips:" : "columns:") + to_string(as.chunks) + ":" +
+                                                          to_string(as.chunk_len) + ":" + to_string(as.sub->size));
+        finish_source(u, pl.decl.str(), body.str(), opt);
+        units.push_back(std::move(u));
+    }
+    return units;
+}
+
 // OUTER_REDUCE: rank 0 sweeps (reductions) with a single parallel sub-nest and no instructions
 // directly at rank 0. Threads own points of the sub-nest and loop over the reduced axis in order.
 bool outer_reduce_applicable(const LoopB &L) {
@@ -4220,7 +4592,10 @@ vector<LaunchUnit> lower_kernel(const LoopB &kernel, const CodegenOptions &opt) 
             const LoopB *sub = split_candidate(*chain[P - 1]);
             int64_t points = 1;
             for (unsigned r = 0; r < P; ++r) points *= chain[r]->size;
-            if (sub != nullptr && points >= kLaneMinPoints && lane_count(points, sub->size) > 1 &&
+            AxisScan as;
+            if (axis_scan_applicable(*chain[P - 1], points, P, opt, as)) {
+                for (LaunchUnit &su : lower_axis_scan(L, P, opt)) units.push_back(std::move(su));
+            } else if (sub != nullptr && points >= kLaneMinPoints && lane_count(points, sub->size) > 1 &&
                 swept_axis_contiguous(*sub, static_cast<int>(P))) {
                 units.push_back(lower_lane_reduce(L, P, opt));
             } else if (sub != nullptr && split_chunks(points, sub->size) > 1) {
@@ -4317,7 +4692,7 @@ vector<int> fuse_tails(const vector<LoopB> &kernels, vector<vector<LaunchUnit>> 
             commutes = !meets(writes[m], reads[j]) && !meets(writes[m], writes[j]) && !meets(reads[m], writes[j]);
         if (!commutes || lowered[k].empty() || into[k] >= 0) continue;
         LaunchUnit &u1 = lowered[k].back();
-        if (u1.tail || u1.sched == Sched::SCAN1D || u1.sched == Sched::SERIAL || u1.sched == Sched::TILE2D ||
+        if (u1.tail || u1.sched == Sched::SCAN1D || u1.sched == Sched::AXIS_SCAN || u1.sched == Sched::SERIAL || u1.sched == Sched::TILE2D ||
             u1.body_core.empty())
             continue;
         u1 = fuse_tail(u1, lowered[j][0]);

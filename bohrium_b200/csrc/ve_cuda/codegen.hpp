@@ -32,6 +32,9 @@
 //                 re-scan with the carry -- each with a fixed block scan (order set by the length).
 //                 With scan_windows, A and C run one group of 2048 chunks at a time (C repeating
 //                 B's steps for its group), so the re-scan reads the group's inputs from L2.
+//   AXIS_SCAN     an accumulate along an axis of an array of two or more dimensions: a thread per
+//                 point (or a warp, when the axis is contiguous), the axis cut into chunks in two
+//                 units (chunk totals, scan) when the points alone are few.
 //   SERIAL        anything else: one thread runs the nest in program order (always correct).
 //   TILE2D        a 2-D map that reads arrays through transposed views (unit stride along the outer
 //                 rank): tiles of (128 bytes / element) rows x 64 columns; each transposed view's
@@ -57,7 +60,7 @@
 namespace bohrium {
 namespace cuda {
 
-enum class Sched { FLAT, GRID_REDUCE, SPLIT_REDUCE, LANE_REDUCE, OUTER_REDUCE, SCAN1D, SERIAL, TILE2D };
+enum class Sched { FLAT, GRID_REDUCE, SPLIT_REDUCE, LANE_REDUCE, OUTER_REDUCE, SCAN1D, SERIAL, TILE2D, AXIS_SCAN };
 
 // Engine-internal opcodes made by contract_multiply_add() (contract.cpp), operands (out, a, b, c):
 //   BH_X_FMA   out = a*b + c      BH_X_FMS   out = a*b - c      BH_X_FNMA  out = c - a*b
@@ -115,10 +118,11 @@ struct LaunchUnit {
     int64_t scratch_bytes_per_tile = 0; // GRID_REDUCE: bytes of partials per tile (all reductions)
     int slot_bytes = 8;         // GRID_REDUCE / SPLIT_REDUCE: bytes of one partial (16 with complex128)
     int64_t chunks = 1;         // SPLIT_REDUCE: chunks of the swept axis; LANE_REDUCE: lanes per point;
-                                // GRID_REDUCE: tiles per work item; SCAN1D: work items of the phase
+                                // GRID_REDUCE: tiles per work item; SCAN1D, AXIS_SCAN: work items of the phase
     int64_t batch_chunks = 0;   // GRID_REDUCE: tiles per work item in a grouped launch (0: chunks)
-    int64_t scan_bytes = 0;     // SCAN1D: its chunk totals and carries and group totals and carries
-    int64_t scan_offset = 0;    // SCAN1D: offset of scan_bytes in the scan arena (set by the plan)
+    int64_t scan_bytes = 0;     // SCAN1D: its chunk totals and carries and group totals and carries;
+                                // AXIS_SCAN: its chunk totals
+    int64_t scan_offset = 0;    // offset of scan_bytes in the scan arena (set by the plan)
     bool scan_gate = false;     // SCAN1D carry unit: one completion counter
     bool single_pass = false;   // SCAN1D in one pass (lower_scan1d_single): chunks = chunk count
     bool no_batch = false;      // always launched alone (its CTAs wait on one another's results)

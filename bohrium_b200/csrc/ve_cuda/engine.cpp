@@ -811,7 +811,7 @@ void EngineCUDA::pack_params(const PlanUnit &pu, const vector<bh_base *> &bases,
             }
             case ParamField::SCRATCH: {
                 void *p = f.i64 == -1              ? static_cast<void *>(err_record)
-                          : u.sched == Sched::SCAN1D ? static_cast<void *>(static_cast<uint8_t *>(scan_arena) + u.scan_offset)
+                          : u.scan_bytes > 0    ? static_cast<void *>(static_cast<uint8_t *>(scan_arena) + u.scan_offset)
                                                      : static_cast<void *>(static_cast<uint8_t *>(scratch) + scratch_off);
                 memcpy(slot, &p, 8);
                 break;
@@ -1330,7 +1330,7 @@ EngineCUDA::FlushPlan EngineCUDA::build_plan(const vector<LoopB> &kernels, const
             vector<LaunchUnit> &units = lowered[kidx];
             int64_t scan_need = 0;
             for (LaunchUnit &u : units) {
-                if (u.sched != Sched::SCAN1D) continue;
+                if (u.scan_bytes == 0) continue;
                 u.scan_offset = plan.scan_bytes;
                 scan_need = max<int64_t>(scan_need, (u.scan_bytes + 255) / 256 * 256);
             }

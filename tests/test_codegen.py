@@ -433,3 +433,22 @@ def test_small_light_grid_reductions_hold_one_variant_per_launch_mode():
     assert units[0]["work"] == 15  # plain work items: one tile each
     _, units = plan(large)
     assert "namespace bh_kg" not in units[0]["source"]
+
+
+def test_accumulates_along_an_axis_lower_to_axis_scan():
+    """An accumulate along an axis of a 2-D array is one AXIS_SCAN unit when the points fill the GPU
+    and two (totals, scan) otherwise; float products and arrays that the nest both reads and changes
+    before the accumulate keep the thread-per-point schedule."""
+    def scheds(make, shape, dtype=np.float32):
+        return [u["sched"] for u in plan(lambda rt: make(bh.array(rt, np.zeros(shape, dtype))))[1]]
+
+    def in_place(a):
+        bh.binary("ADD", a, 1.0, out=a)
+        return [a, a.cumsum(1)]
+
+    assert scheds(lambda a: [a.cumsum(1)], (6000, 40)) == ["axis_scan"]
+    assert scheds(lambda a: [a.cumsum(1)], (3, 100_000)) == ["axis_scan", "axis_scan"]
+    assert scheds(lambda a: [a.cumsum(0)], (100_000, 3)) == ["axis_scan", "axis_scan"]
+    assert scheds(lambda a: [a.cumprod(1)], (3, 100_000), np.int32) == ["axis_scan", "axis_scan"]
+    assert "axis_scan" not in scheds(lambda a: [a.cumprod(1)], (3, 100_000))
+    assert "axis_scan" not in scheds(in_place, (3, 100_000))

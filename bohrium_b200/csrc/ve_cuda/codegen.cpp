@@ -48,7 +48,7 @@ int64_t LaunchUnit::work_items() const {
             const int64_t tiles = (cols + kReduceTile - 1) / kReduceTile;
             return (tiles + chunks - 1) / chunks;  // chunks: tiles per work item
         }
-        case Sched::SPLIT_REDUCE: return (rows * cols + kThreads - 1) / kThreads * chunks;
+        case Sched::SPLIT_REDUCE: return (rows * cols + V - 1) / V * chunks;  // V: points per CTA
         case Sched::LANE_REDUCE: {
             const int64_t per = kThreads / chunks;
             return (rows * cols + per - 1) / per;
@@ -85,7 +85,8 @@ int64_t LaunchUnit::counters_needed() const {
         own = chunks + (chunks + 7) / 8 + (chunks + 255) / 256 + ngroups + 1 + 3;
     }
     if (sched == Sched::GRID_REDUCE) own = 1;
-    if (sched == Sched::SPLIT_REDUCE) own = (rows * cols + kThreads - 1) / kThreads;
+    if (sched == Sched::SPLIT_REDUCE)  // per block of points: its segments of chunks, and the block
+        own = (rows * cols + V - 1) / V * ((chunks + kSplitSegment - 1) / kSplitSegment + 1);
     if (sched == Sched::SCAN1D && scan_gate) own = 1;
     return tail ? own + 1 : own;  // the tail's completion counter follows
 }
@@ -1370,6 +1371,39 @@ void hoist_views(Emitter &em, const LoopB &inner, int axis, ostream &out, int in
     em.hoist_axis = axis;
 }
 
+// Running pointers of `views` along loop index i<axis> (hoist_views has been called for them): qp<k>
+// points at the element of index `first` and advances by `step` indices, so a load costs one
+// pointer addition instead of a 64-bit multiply and two additions.
+bool running_pointers(Emitter &em, const vector<bh_view> &views, int axis, const string &first, const string &step,
+                      ostream &out, int ind) {
+    for (const bh_view &v : views)
+        if (!em.hoisted.count(em.sym.view_id.at(v))) return false;
+    const string sp(static_cast<size_t>(ind), ' '), i = "i" + to_string(axis);
+    for (size_t k = 0; k < views.size(); ++k) {
+        const string T = cuda_type(views[k].base->dtype()), hp = em.hoisted.at(em.sym.view_id.at(views[k]));
+        const string term = em.axis_term(views[k], axis);
+        out << sp << "const " << T << " *qp" << k << "; bh_i64 qs" << k << ";\n";
+        out << sp << "{ const bh_i64 " << i << " = " << first << "; qp" << k << " = " << hp << " + (" << term << "); }\n";
+        out << sp << "{ const bh_i64 " << i << " = " << step << "; qs" << k << " = " << term << "; }\n";
+    }
+    return true;
+}
+
+// As emit_preload, from running pointers, which end up at the next block's first element.
+void emit_preload_running(const vector<bh_view> &views, int V, const string &index_decl, const string &guard,
+                          Scope &scope, ostream &out, int ind) {
+    const string sp(static_cast<size_t>(ind), ' ');
+    for (size_t k = 0; k < views.size(); ++k)
+        out << sp << cuda_type(views[k].base->dtype()) << " pl" << k << "[" << V << "];\n";
+    out << "#pragma unroll\n";
+    out << sp << "for (int j = 0; j < " << V << "; ++j) {\n";
+    if (!guard.empty()) out << sp << "    " << index_decl << "\n" << sp << "    if (" << guard << ") break;\n";
+    for (size_t k = 0; k < views.size(); ++k)
+        out << sp << "    pl" << k << "[j] = *qp" << k << "; qp" << k << " += qs" << k << ";\n";
+    out << sp << "}\n";
+    for (size_t k = 0; k < views.size(); ++k) scope.repl[ViewKey(views[k])] = "pl" + to_string(k) + "[j]";
+}
+
 // Emit the register arrays and the load loop of `views` for V elements per thread; element j has
 // index `idx_init(j)` (a statement defining the innermost loop index). With `guard` the loads
 // stop at the loop bound. Registers the replacements in `scope`.
@@ -2429,6 +2463,50 @@ LaunchUnit lower_lane_reduce(const LoopB &loop, unsigned P, const CodegenOptions
     return u;
 }
 
+// SPLIT_REDUCE: a CTA's threads are `block` neighbouring points x `groups` rows of the swept axis
+// (256 points and one group when there are enough points; otherwise all points side by side, so a
+// narrow array keeps its threads; one point and 256 groups when the swept axis is contiguous, so
+// neighbouring threads read neighbouring elements either way). The rows are dealt to the groups of
+// all chunks in turn; each thread folds its rows in order, kSplitUnroll loads ahead, and a
+// shared-memory tree folds the groups. The chunk partials are folded in two levels (see emit_gate
+// below), so the last fold stays short. The order depends on the shapes only.
+// Bound by the bytes in flight (loads take about 1.3 us under load): four CTAs of 256 threads fit
+// an SM at up to 64 registers a thread, and one wave of them is aimed at -- 594 CTAs instead of 588 cost a
+// second wave and a third of the time. Sums over the rows of float64 tables, before (one thread
+// per point and chunk, all partials folded by one CTA) and here: 500003 x 50 750 and 49 us,
+// 20000 x 1500 101 and 54 us, 4000 x 4099 57 and 37 us, 300 x 100000 51 and 54 us; along the rows
+// of 5 x 5000000 6.5 ms and 61 us. 4 or 16 loads ahead, six CTAs per SM, chunks of
+// consecutive rows and a ring of cp.async copies measured slower.
+constexpr int kSplitUnroll = 8;
+constexpr int64_t kSplitCtas = 148 * 4;    // CTAs aimed at
+constexpr int64_t kSplitFewChunks = 8;
+struct SplitShape {
+    int64_t block = kThreads, groups = 1, chunks = 1;
+};
+SplitShape split_shape(int64_t points, int64_t len, bool contiguous) {
+    SplitShape s;
+    s.block = contiguous ? 1 : max<int64_t>(1, min<int64_t>(points, kThreads));
+    s.groups = kThreads / s.block;
+    const int64_t blocks = max<int64_t>(1, (points + s.block - 1) / s.block);
+    const int64_t most = max<int64_t>(1, len / (kSplitMinChunk * s.groups));
+    // Few blocks: one full wave of CTAs. Many blocks: the number of chunks (up to kSplitFewChunks)
+    // that fills its last wave best, the smallest within 2 % of it.
+    int64_t want = max<int64_t>(1, kSplitCtas / blocks);
+    if (want < kSplitFewChunks) {
+        double best = 0;
+        for (int64_t c = 1; c <= kSplitFewChunks; ++c) {
+            const int64_t total = c * blocks, waves = (total + kSplitCtas - 1) / kSplitCtas;
+            const double fill = static_cast<double>(total) / static_cast<double>(waves * kSplitCtas);
+            if (fill > best + 0.02) {
+                best = fill;
+                want = c;
+            }
+        }
+    }
+    s.chunks = max<int64_t>(1, min(want, most));
+    return s;
+}
+
 LaunchUnit lower_split_reduce(const LoopB &loop, unsigned P, const CodegenOptions &opt) {
     LaunchUnit u;
     u.sched = Sched::SPLIT_REDUCE;
@@ -2451,16 +2529,21 @@ LaunchUnit lower_split_reduce(const LoopB &loop, unsigned P, const CodegenOption
     u.rows = rows;
     u.cols = inner.size;
     const int64_t points = rows * inner.size;
-    u.chunks = split_chunks(points, sub.size);
-    const int64_t chunk_len = (sub.size + u.chunks - 1) / u.chunks;
+    const SplitShape shape = split_shape(points, sub.size, swept_axis_contiguous(sub, static_cast<int>(P)));
+    u.chunks = shape.chunks;
+    u.V = static_cast<int>(shape.block);
     for (const InstrPtr &r : reds)
-        u.red_orders.emplace_back(r->origin_id, "split:" + to_string(u.chunks) + ":" + to_string(chunk_len) + ":" +
+        u.red_orders.emplace_back(r->origin_id, "split:" + to_string(shape.chunks) + ":" + to_string(shape.groups) + ":" +
                                                     to_string(sub.size));
+    int64_t half = 1;  // the largest power of two below `groups` (1 for one group)
+    while (half * 2 < shape.groups) half *= 2;
     ParamLayout pl;
     add_common_fields(sym, pl, opt);
     pl.add(work_field(points), "bh_i64", "points");
-    pl.add(work_field(u.chunks), "bh_i64", "chunks");
-    pl.add(work_field(chunk_len), "bh_i64", "chunk_len");
+    pl.add(work_field(shape.chunks), "bh_i64", "chunks");
+    pl.add(work_field(shape.block), "bh_i64", "block");
+    pl.add(work_field(shape.groups), "bh_i64", "groups");
+    pl.add(work_field(half), "bh_i64", "half");
     pl.add(work_field(u.work_items()), "bh_i64", "work");
     ParamField fs{ParamField::SCRATCH};
     pl.add(fs, "unsigned char*", "scratch");
@@ -2476,13 +2559,36 @@ LaunchUnit lower_split_reduce(const LoopB &loop, unsigned P, const CodegenOption
         idents.push_back(constant_literal(jitk::sweep_identity(reds[k]->opcode, t)));
         em.external_acc[ViewKey(reds[k]->operand[0])] = "pacc" + to_string(k);
     }
-    const int sub_lid = sym.loop_id.at(&sub);
+    u.slot_bytes = red_slot_bytes(reds);
+    const string n_sub = "(bh_i64)p.n" + to_string(sym.loop_id.at(&sub)), ix = "i" + to_string(P);
+    // Folds the groups' values of each point into group 0, by halving the groups.
+    for (size_t k = 0; k < reds.size(); ++k) {
+        const string &T = ctypes[k];
+        body << "__device__ __forceinline__ " << T << " bh_groups" << k << "(const P &p, " << T << " v, unsigned char *sm) {\n";
+        body << "    if (p.groups == 1) return v;\n";
+        body << "    const int block = (int)p.block, groups = (int)p.groups, g = threadIdx.x / block;\n";
+        body << "    " << T << " *x = (" << T << " *)sm + threadIdx.x;\n";
+        body << "    *x = v;\n";
+        body << "    __syncthreads();\n";
+        body << "    for (int s = (int)p.half; s > 0; s >>= 1) {\n";
+        body << "        if (g < s && g + s < groups) {\n";
+        body << "            const " << T << " y = x[s * block];\n";
+        body << "            v = " << reduce_expr(reds[k]->opcode, "v", "y") << ";\n";
+        body << "            *x = v;\n";
+        body << "        }\n";
+        body << "        __syncthreads();\n";
+        body << "    }\n";
+        body << "    return v;\n";
+        body << "}\n";
+    }
     body << "__device__ void bh_work(const P &p, bh_i64 w) {\n";
     body << pointer_locals(sym);
     body << "    __shared__ bool am_last;\n";
+    body << "    __shared__ alignas(16) unsigned char group_sm[" << kThreads * u.slot_bytes << "];\n";
     body << "    const bh_i64 pb = w / p.chunks, chunk = w - pb * p.chunks;\n";
-    body << "    const bh_i64 pt = pb * " << kThreads << " + threadIdx.x;\n";
-    u.slot_bytes = red_slot_bytes(reds);
+    body << "    const int block = (int)p.block, groups = (int)p.groups, g = threadIdx.x / block;\n";
+    body << "    const bh_i64 pt = pb * block + (threadIdx.x - g * block);\n";
+    body << "    const bool active = g < groups && pt < p.points;\n";
     for (size_t k = 0; k < reds.size(); ++k)
         body << "    " << ctypes[k] << "* part" << k << " = (" << ctypes[k] << "*)(p.scratch + " << u.slot_bytes * k
              << " * p.chunks * p.points);\n";
@@ -2500,64 +2606,104 @@ LaunchUnit lower_split_reduce(const LoopB &loop, unsigned P, const CodegenOption
         }
         body << sp << "(void)rem;\n";
     };
-    body << "    if (pt < p.points) {\n";
+    for (size_t k = 0; k < reds.size(); ++k) body << "    " << ctypes[k] << " pacc" << k << " = " << idents[k] << ";\n";
+    body << "    if (active) {\n";
     decompose(8);
     {
         Scope scope;
         declare_chain_temps(em, sym, scope, chain, P, body, 8);
-        for (size_t k = 0; k < reds.size(); ++k) body << "        " << ctypes[k] << " pacc" << k << " = " << idents[k] << ";\n";
-        body << "        const bh_i64 lo = chunk * p.chunk_len;\n";
-        body << "        const bh_i64 hi = min(lo + p.chunk_len, (bh_i64)p.n" << sub_lid << ");\n";
-        body << "/*@unroll@*/\n";  // the autotuner may put an unroll pragma here
-        body << "        for (bh_i64 i" << P << " = lo; i" << P << " < hi; ++i" << P << ") {\n";
-        Scope s1;
-        s1.parent = &scope;
-        em.write_body(sub, s1, 12);
-        body << "        }\n";
-        for (size_t k = 0; k < reds.size(); ++k)
-            body << "        part" << k << "[chunk * p.points + pt] = pacc" << k << ";\n";
+        body << "        const bh_i64 step = p.chunks * groups, hi = " << n_sub << ";\n";
+        hoist_views(em, sub, static_cast<int>(P), body, 8);
+        const vector<bh_view> pre = preloadable_views(sub, L, sym);
+        const string idx = "const bh_i64 " + ix + " = base + j * step;";
+        const bool running = running_pointers(em, pre, static_cast<int>(P), "chunk * groups + g", "step", body, 8);
+        body << "        for (bh_i64 base = chunk * groups + g; base < hi; base += " << kSplitUnroll << " * step) {\n";
+        for (int path = 0; path < 2; ++path) {
+            // path 0: every element of the block lies in the chunk; path 1: the last block.
+            body << (path == 0 ? "            if (base + " + to_string(kSplitUnroll - 1) + " * step < hi) {\n"
+                               : "            } else {\n");
+            const string guard = path == 0 ? "" : ix + " >= hi";
+            Scope s1;
+            s1.parent = &scope;
+            if (running) {
+                emit_preload_running(pre, kSplitUnroll, idx, guard, s1, body, 16);
+            } else {
+                emit_preload(em, pre, kSplitUnroll, idx, guard, s1, body, 16);
+            }
+            body << "#pragma unroll\n";
+            body << "                for (int j = 0; j < " << kSplitUnroll << "; ++j) {\n";
+            body << "                    " << idx << "\n";
+            if (path == 1) body << "                    if (" << guard << ") break;\n";
+            em.write_body(sub, s1, 20);
+            body << "                }\n";
+        }
+        body << "            }\n        }\n";
+        em.hoisted.clear();
     }
     body << "    }\n";
-    body << "    __syncthreads();\n";
-    body << "    if (threadIdx.x == 0) {\n";
-    body << "        am_last = bh_arrive((unsigned*)(p.counter + pb)) == (unsigned)(p.chunks - 1);\n";
-    body << "    }\n";
-    body << "    __syncthreads();\n";
-    body << "    if (!am_last) return;\n";
-    body << "    bh_acquire();\n";
-    body << "    if (threadIdx.x == 0) p.counter[pb] = 0u;\n";
-    body << "    if (pt >= p.points) return;\n";
-    {
-        decompose(4);
-        Scope scope;
-        declare_chain_temps(em, sym, scope, chain, P - 1, body, 4);
-        // The chunk partials were written by other CTAs (made visible by the fence and the
-        // counter): read them through L2 (ld.global.cg), eight loads in flight, folded in chunk
-        // order.
+    for (size_t k = 0; k < reds.size(); ++k) {
+        body << "    pacc" << k << " = bh_groups" << k << "(p, pacc" << k << ", group_sm);\n";
+        body << "    if (active && g == 0) part" << k << "[chunk * p.points + pt] = pacc" << k << ";\n";
+    }
+    // The CTA that finishes a segment of kSplitSegment chunks last folds its partials in chunk order
+    // into the segment's first slot, and the one that finishes the last segment folds the segments:
+    // two short folds instead of one long one. The partials were written by other CTAs (made
+    // visible by the fence and the counter): they are read through L2 (ld.global.cg), eight loads
+    // in flight; group g takes every groups-th partial from g on.
+    auto emit_gate = [&](const string &counter, const string &arrivals) {
+        body << "    __syncthreads();\n";
+        body << "    if (threadIdx.x == 0) am_last = bh_arrive((unsigned*)(" << counter << ")) == (unsigned)(" << arrivals << " - 1);\n";
+        body << "    __syncthreads();\n";
+        body << "    if (!am_last) return;\n";
+        body << "    bh_acquire();\n";
+        body << "    if (threadIdx.x == 0) *(" << counter << ") = 0u;\n";
+    };
+    auto emit_fold = [&](const string &first, const string &count, const string &stride) {
         for (size_t k = 0; k < reds.size(); ++k) {
             const string acc = "pacc" + to_string(k), T = ctypes[k];
-            body << "    " << T << " " << acc << " = " << idents[k] << ";\n";
-            body << "    {\n";
-            body << "        bh_i64 c = 0;\n";
-            body << "        for (; c + 8 <= p.chunks; c += 8) {\n";
+            const string at = "part" + to_string(k) + " + (" + first + " + (c";
+            body << "    " << acc << " = " << idents[k] << ";\n";
+            body << "    if (active) {\n";
+            body << "        bh_i64 c = g;\n";
+            body << "        for (; c + 7 * groups < " << count << "; c += 8 * groups) {\n";
             body << "            " << T << " x[8];\n";
             body << "#pragma unroll\n";
-            body << "            for (int j = 0; j < 8; ++j) x[j] = bh_ldcg(part" << k << " + (c + j) * p.points + pt);\n";
+            body << "            for (int j = 0; j < 8; ++j) x[j] = bh_ldcg(" << at << " + j * groups) * " << stride
+                 << ") * p.points + pt);\n";
             body << "#pragma unroll\n";
             body << "            for (int j = 0; j < 8; ++j) " << acc << " = " << reduce_expr(reds[k]->opcode, acc, "x[j]")
                  << ";\n";
             body << "        }\n";
-            body << "        for (; c < p.chunks; ++c) {\n";
-            body << "            const " << T << " x = bh_ldcg(part" << k << " + c * p.points + pt);\n";
+            body << "        for (; c < " << count << "; c += groups) {\n";
+            body << "            const " << T << " x = bh_ldcg(" << at << ") * " << stride << ") * p.points + pt);\n";
             body << "            " << acc << " = " << reduce_expr(reds[k]->opcode, acc, "x") << ";\n";
             body << "        }\n";
             body << "    }\n";
+            body << "    " << acc << " = bh_groups" << k << "(p, " << acc << ", group_sm);\n";
         }
+    };
+    body << "    const bh_i64 seg = chunk / " << kSplitSegment << ", nseg = (p.chunks + " << kSplitSegment - 1 << ") / "
+         << kSplitSegment << ";\n";
+    body << "    const bh_i64 seg0 = seg * " << kSplitSegment << ", in_seg = min((bh_i64)" << kSplitSegment
+         << ", p.chunks - seg0);\n";
+    emit_gate("p.counter + pb * (nseg + 1) + seg", "in_seg");
+    emit_fold("seg0", "in_seg", "1");
+    body << "    if (nseg > 1) {\n";
+    for (size_t k = 0; k < reds.size(); ++k)
+        body << "    if (active && g == 0) part" << k << "[seg0 * p.points + pt] = pacc" << k << ";\n";
+    emit_gate("p.counter + pb * (nseg + 1) + nseg", "nseg");
+    emit_fold("0", "nseg", to_string(kSplitSegment));
+    body << "    }\n";
+    body << "    if (active && g == 0) {\n";
+    decompose(8);
+    {
+        Scope scope;
+        declare_chain_temps(em, sym, scope, chain, P - 1, body, 8);
         // Instructions after the swept sub-loop, then the reduction outputs.
         for (const bh_base *b : em.sorted_temps(inner)) {
             if (sym.temps.count(b) && !scope.is_tmp(b)) {
                 scope.tmps.insert(b);
-                body << "    " << cuda_type(b->dtype()) << " t" << sym.base_index(b) << ";\n";
+                body << "        " << cuda_type(b->dtype()) << " t" << sym.base_index(b) << ";\n";
             }
         }
         bool after = false;
@@ -2566,13 +2712,15 @@ LaunchUnit lower_split_reduce(const LoopB &loop, unsigned P, const CodegenOption
                 after = true;
                 continue;
             }
-            if (after) em.write_instr(*b.getInstr(), scope, 4);
+            if (after) em.write_instr(*b.getInstr(), scope, 8);
         }
         for (size_t k = 0; k < reds.size(); ++k) {
             if (sym.temps.count(reds[k]->operand[0].base)) continue;
-            body << "    " << em.array_ref(reds[k]->operand[0], reds[k]->sweep_axis()) << " = pacc" << k << ";\n";
+            body << "        " << em.array_ref(reds[k]->operand[0], reds[k]->sweep_axis()) << " = pacc" << k << ";\n";
         }
     }
+    body << "    }\n";
+    body << "    __syncthreads();\n";  // the next work item writes the shared memory again
     body << "}\n" << kWrappers;
     u.fields = pl.fields;
     u.algorithmic_bytes = unit_bytes(sym, vector<const Block *>{&holder});

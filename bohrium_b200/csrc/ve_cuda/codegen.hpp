@@ -15,9 +15,9 @@
 //                 for bit.
 //   SPLIT_REDUCE  a FLAT nest with few parallel points whose innermost threaded loop holds one
 //                 swept sub-loop (axis reductions such as max over the rows of a 2-D array): the
-//                 swept axis is cut into chunks so that ~600K threads work at once; each thread folds
-//                 its chunk in order, and the last CTA of each 256-point block folds the chunk
-//                 partials in chunk order (deterministic) and runs the instructions that follow.
+//                 swept axis is cut into chunks, and a CTA with fewer than 256 points into groups, so
+//                 that one wave of CTAs works on it; the partials are folded in a fixed order by the
+//                 CTAs that finish last, which also run the instructions that follow.
 //   LANE_REDUCE   the SPLIT_REDUCE structure when the swept axis is contiguous and there are
 //                 enough points: C (power of two <= 256, from the shapes) lanes of one CTA share a
 //                 point, lane c folds elements c, c+C, ... (coalesced), and a fixed shuffle tree
@@ -84,6 +84,7 @@ const char *sched_name(Sched s);
 constexpr int kThreads = 256;      // threads per CTA for every schedule
 constexpr int kReduceV = 8;        // elements per thread per tile in GRID_REDUCE
 constexpr int64_t kReduceTile = kThreads * kReduceV;
+constexpr int64_t kSplitSegment = 16; // chunk partials folded together in SPLIT_REDUCE
 constexpr int64_t kScanChunk = 4096; // elements per chunk in SCAN1D
 
 // One 8-byte slot (or two for 16-byte constants) of the kernel parameter struct.
@@ -146,7 +147,7 @@ struct LaunchUnit {
     int64_t elements = 0;
 
     // Summation order of the sweeps this unit reduces across threads, by origin id: "tree:<n>"
-    // (GRID_REDUCE) or "split:<chunks>:<chunk length>:<n>" (SPLIT_REDUCE). Every other sweep is
+    // (GRID_REDUCE) or "split:<chunks>:<groups>:<n>" (SPLIT_REDUCE). Every other sweep is
     // folded by one thread in index order ("seq"), whatever the schedule.
     std::vector<std::pair<int64_t, std::string>> red_orders;
 };

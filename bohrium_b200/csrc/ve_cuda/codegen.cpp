@@ -1452,10 +1452,30 @@ string word_copy(const string &dst, const string &src, int bytes) {
     return ss.str();
 }
 
+// Where the 4 elements of a thread lie. Plain: in one row of the innermost rank, at cbase .. cbase
+// + 3. Collapsed (rows that would leave many of a CTA's threads idle): consecutive in the index
+// space of the two innermost ranks taken row after row, element j at (rr[j], cc[j]); a view whose
+// rows follow each other without gaps is still moved as words.
+struct FlatIndex {
+    bool collapsed = false;
+    int axis = 0;          // the innermost rank
+    string n_inner;        // its length
+    // Declares the loop indices of element `j`.
+    string decl(const string &j) const {
+        const string iv = "i" + to_string(axis);
+        if (!collapsed) return "const bh_i64 " + iv + " = cbase + " + j + ";";
+        return "const bh_i64 i" + to_string(axis - 1) + " = rr[" + j + "], " + iv + " = cc[" + j + "];";
+    }
+    bool words(const bh_view &v, const Symbols &sym) const {
+        if (!unit_stride_view(v, axis, sym)) return false;
+        return !collapsed || v.stride[axis - 1] == v.shape[axis];
+    }
+};
+
 void emit_flat_vector(Symbols &sym, ostream &body, const CodegenOptions &opt, const LoopB &inner,
                       const vector<const LoopB *> &chain, unsigned P, const vector<bh_view> &pre, int64_t per,
-                      const string &n_inner, const string &iv) {
-    const int axis = static_cast<int>(P) - 1;
+                      const FlatIndex &fi) {
+    const string n_total = fi.collapsed ? "p.cells" : fi.n_inner;
     // Written views that can be stored as words: outputs of elementwise instructions of `inner`,
     // unit stride, their base written and read in the kernel through this one view only.
     map<const bh_base *, set<ViewKey>> touched;
@@ -1470,18 +1490,34 @@ void emit_flat_vector(Symbols &sym, ostream &body, const CodegenOptions &opt, co
             op == BH_COND_SCATTER || i->operand.empty())
             continue;
         const bh_view &v = i->operand[0];
-        if (!unit_stride_view(v, axis, sym) || sym.always_array.count(v.base) || touched[v.base].size() != 1) continue;
+        if (!fi.words(v, sym) || sym.always_array.count(v.base) || touched[v.base].size() != 1) continue;
         if (seen_out.insert(ViewKey(v)).second) outs.push_back(v);
     }
     vector<bool> vec_pre(pre.size());
-    for (size_t k = 0; k < pre.size(); ++k) vec_pre[k] = unit_stride_view(pre[k], axis, sym);
+    for (size_t k = 0; k < pre.size(); ++k) vec_pre[k] = fi.words(pre[k], sym);
     Emitter em(sym, body, opt);
     body << "    const bh_i64 cbase = chunk * " << per << " + threadIdx.x * 4;\n";
-    body << "    if ((chunk + 1) * " << per << " <= " << n_inner << ") {\n";
+    if (fi.collapsed) {
+        body << "    const unsigned nb = (unsigned)" << fi.n_inner << ", row0 = (unsigned)(chunk * " << per << ") / nb;\n";
+        body << "    const unsigned loc = (unsigned)(chunk * " << per << ") - row0 * nb + threadIdx.x * 4, lr = loc / nb;\n";
+        body << "    unsigned rr[4] = {row0 + lr}, cc[4] = {loc - lr * nb};\n";
+        body << "#pragma unroll\n";
+        body << "    for (int j = 1; j < 4; ++j) {\n";
+        body << "        const bool wrap = cc[j - 1] + 1u == nb;\n";
+        body << "        rr[j] = rr[j - 1] + (wrap ? 1u : 0u);\n";
+        body << "        cc[j] = wrap ? 0u : cc[j - 1] + 1u;\n";
+        body << "    }\n";
+    }
+    // Full chunks run without bounds checks (collapsed: threads whose 4 elements all exist).
+    if (fi.collapsed) {
+        body << "    if (cbase + 4 <= " << n_total << ") {\n";
+    } else {
+        body << "    if ((chunk + 1) * " << per << " <= " << n_total << ") {\n";
+    }
     // Word alignment of every word-moved view at element cbase.
     body << "        bool vec = true;\n";
     body << "        {\n";
-    body << "            const bh_i64 " << iv << " = cbase;\n";
+    body << "            " << fi.decl("0") << "\n";
     auto align_check = [&](const bh_view &v) {
         const int bytes = min(16, 4 * static_cast<int>(bh_type_size(v.base->dtype())));
         body << "            vec = vec && (((unsigned long long)&" << em.array_ref(v) << ") & " << bytes - 1 << "ull) == 0;\n";
@@ -1497,7 +1533,7 @@ void emit_flat_vector(Symbols &sym, ostream &body, const CodegenOptions &opt, co
         const int bytes = 4 * static_cast<int>(bh_type_size(pre[k].base->dtype()));
         if (vec_pre[k]) {
             body << "        if (vec) {\n";
-            body << "            const bh_i64 " << iv << " = cbase;\n";
+            body << "            " << fi.decl("0") << "\n";
             body << "            " << word_copy("pl" + to_string(k), "&" + em.array_ref(pre[k]), bytes) << "\n";
             body << "        } else {\n";
         } else {
@@ -1505,7 +1541,7 @@ void emit_flat_vector(Symbols &sym, ostream &body, const CodegenOptions &opt, co
         }
         body << "#pragma unroll\n";
         body << "            for (int j = 0; j < 4; ++j) {\n";
-        body << "                const bh_i64 " << iv << " = cbase + j;\n";
+        body << "                " << fi.decl("j") << "\n";
         body << "                pl" << k << "[j] = " << em.array_ref(pre[k]) << ";\n";
         body << "            }\n";
         body << "        }\n";
@@ -1517,7 +1553,7 @@ void emit_flat_vector(Symbols &sym, ostream &body, const CodegenOptions &opt, co
     }
     body << "#pragma unroll\n";
     body << "        for (int j = 0; j < 4; ++j) {\n";
-    body << "            const bh_i64 " << iv << " = cbase + j;\n";
+    body << "            " << fi.decl("j") << "\n";
     {
         Emitter eb(sym, body, opt);
         declare_chain_temps(eb, sym, scope, chain, P - 1, body, 12);
@@ -1527,12 +1563,12 @@ void emit_flat_vector(Symbols &sym, ostream &body, const CodegenOptions &opt, co
     for (size_t k = 0; k < outs.size(); ++k) {
         const int bytes = 4 * static_cast<int>(bh_type_size(outs[k].base->dtype()));
         body << "        if (vec) {\n";
-        body << "            const bh_i64 " << iv << " = cbase;\n";
+        body << "            " << fi.decl("0") << "\n";
         body << "            " << word_copy("&" + em.array_ref(outs[k]), "so" + to_string(k), bytes) << "\n";
         body << "        } else {\n";
         body << "#pragma unroll\n";
         body << "            for (int j = 0; j < 4; ++j) {\n";
-        body << "                const bh_i64 " << iv << " = cbase + j;\n";
+        body << "                " << fi.decl("j") << "\n";
         body << "                " << em.array_ref(outs[k]) << " = so" << k << "[j];\n";
         body << "            }\n";
         body << "        }\n";
@@ -1541,14 +1577,36 @@ void emit_flat_vector(Symbols &sym, ostream &body, const CodegenOptions &opt, co
     {
         Scope s1;
         Emitter eb(sym, body, opt);
+        if (fi.collapsed) body << "#pragma unroll\n";
         body << "        for (int j = 0; j < 4; ++j) {\n";
-        body << "            const bh_i64 " << iv << " = cbase + j;\n";
-        body << "            if (" << iv << " >= " << n_inner << ") break;\n";
+        body << "            if (cbase + j >= " << n_total << ") break;\n";
+        body << "            " << fi.decl("j") << "\n";
         declare_chain_temps(eb, sym, s1, chain, P - 1, body, 12);
         eb.write_body(inner, s1, 12);
         body << "        }\n";
     }
     body << "    }\n";
+}
+
+// Whether a map walks its two innermost ranks as one (FlatIndex::collapsed): rows of `cols` elements
+// that keep less than this share of a CTA's threads busy in chunks of `per`, and large maps with
+// 8-byte elements whose rows end in a partial chunk. At 500003 x 50 a division by a row vector took
+// 532 (float32) and 828 us (float64) row by row and takes 64 and 76 us, at 100000 x 300 128 and 201
+// against 74 and 89 us. Longer float64 rows: 20000 x 1023 110 against 64 us, 20000 x 1500 106 against
+// 88 us, 4000 x 4099 79 against 54 us; float32 rows there lose as much as they gain (20000 x 1500
+// 65 against 74 us, a column vector 112 against 84 us; 4000 x 4099 38 against 46 us): the index
+// arithmetic and the scalar loads of views with gaps cost more than the idle threads.
+constexpr double kFlatRowUse = 0.7;
+constexpr int64_t kFlatWideCells = int64_t{1} << 20;
+bool flat_collapses(const LoopB &L, int64_t row_count, int64_t cols, int64_t per) {
+    const int64_t covered = (cols + per - 1) / per * per;
+    if (cols <= 0 || row_count * cols >= (int64_t{1} << 31)) return false;  // 32-bit index arithmetic
+    if (static_cast<double>(cols) < kFlatRowUse * static_cast<double>(covered)) return true;
+    if (cols == covered || row_count * cols < kFlatWideCells) return false;
+    for (const InstrPtr &i : jitk::all_instr(L))
+        for (const bh_view &v : i->operand)
+            if (!v.isConstant() && bh_type_size(v.base->dtype()) >= 8) return true;
+    return false;
 }
 
 // Elements of a map small enough to run in another kernel's tail: a few values computed from a
@@ -1570,9 +1628,22 @@ LaunchUnit lower_flat(const LoopB &loop, unsigned P, const CodegenOptions &opt) 
     u.rows = rows;
     u.cols = inner.size;
     const int64_t per = static_cast<int64_t>(kThreads) * u.V;
-    const int64_t chunks = (u.cols + per - 1) / per;
+    int64_t chunks = (u.cols + per - 1) / per;
+    const bool vector_form = u.V == 4 && opt.vector_access && !opt.bounds_check;
+    FlatIndex fi;
+    fi.axis = static_cast<int>(P) - 1;
+    fi.n_inner = "p.n" + to_string(sym.loop_id.at(&inner));
+    fi.collapsed = vector_form && P >= 2 && flat_collapses(L, chain[P - 2]->size, u.cols, per);
+    const unsigned outer_ranks = fi.collapsed ? P - 2 : P - 1;  // ranks walked row by row
+    if (fi.collapsed) {
+        rows /= chain[P - 2]->size;
+        u.rows = rows;
+        u.cols *= chain[P - 2]->size;
+        chunks = (u.cols + per - 1) / per;
+    }
     ParamLayout pl;
     add_common_fields(sym, pl, opt);
+    if (fi.collapsed) pl.add(work_field(u.cols), "bh_i64", "cells");
     pl.add(work_field(chunks), "bh_i64", "chunks");
     pl.add(work_field(rows * chunks), "bh_i64", "work");
 
@@ -1583,7 +1654,7 @@ LaunchUnit lower_flat(const LoopB &loop, unsigned P, const CodegenOptions &opt) 
     body << "    const bh_i64 row = w / p.chunks;\n";
     body << "    const bh_i64 chunk = w - row * p.chunks;\n";
     body << "    bh_i64 rem = row;\n";
-    for (int r = static_cast<int>(P) - 2; r >= 0; --r) {
+    for (int r = static_cast<int>(outer_ranks) - 1; r >= 0; --r) {
         const int lid = sym.loop_id.at(chain[r]);
         if (r == 0) {
             body << "    const bh_i64 i0 = rem;\n";
@@ -1595,7 +1666,6 @@ LaunchUnit lower_flat(const LoopB &loop, unsigned P, const CodegenOptions &opt) 
     const vector<bh_view> pre =
         u.V > 1 && !(heavy_body(inner) && !opt.preload_heavy) ? preloadable_views(inner, L, sym) : vector<bh_view>{};
     const string n_inner = "p.n" + to_string(sym.loop_id.at(&inner));
-    const string iv = "i" + to_string(P - 1);
     // A tiny map (at most kFlatTailElements elements) can also run in the tail of the kernel
     // before it, by the CTA that finishes that kernel last (fuse_tails): one CTA runs every work
     // item in turn. Elementwise results do not depend on which thread computes them. (bh_tail is
@@ -1605,8 +1675,8 @@ LaunchUnit lower_flat(const LoopB &loop, unsigned P, const CodegenOptions &opt) 
                                               "    for (bh_i64 w = 0; w < p.work; ++w) bh_work(p, w);\n"
                                               "}\n";
     u.tail_capable = !opt.bounds_check && rows * u.cols <= kFlatTailElements;
-    if (u.V == 4 && opt.vector_access && !opt.bounds_check) {
-        emit_flat_vector(sym, body, opt, inner, chain, P, pre, per, n_inner, iv);
+    if (vector_form) {
+        emit_flat_vector(sym, body, opt, inner, chain, P, pre, per, fi);
         body << "}\n" << tail_fn << kWrappers;
         u.fields = pl.fields;
         u.algorithmic_bytes = unit_bytes(sym, vector<const Block *>{&holder});

@@ -1431,6 +1431,18 @@ void emit_preload(Emitter &em, const vector<bh_view> &views, int V, const string
 // strides, element by element. The written values stay in registers until the words are stored,
 // and later reads of them in the element code use the registers. Every element is computed by the
 // same statements either way, so the results do not depend on the path.
+// True when the instructions of `L` read view `v`'s array before they write it: an update in place,
+// whose register copy has to start from the array's value.
+bool read_before_written(const LoopB &L, const bh_view &v) {
+    for (const InstrPtr &i : jitk::all_instr(L)) {
+        if (bh_opcode_is_system(i->opcode)) continue;
+        for (size_t o = 1; o < i->operand.size(); ++o)
+            if (!i->operand[o].isConstant() && i->operand[o].base == v.base) return true;
+        if (!i->operand.empty() && !i->operand[0].isConstant() && i->operand[0].base == v.base) return false;
+    }
+    return false;
+}
+
 // Views that can be moved as words: unit stride along the innermost rank `axis`, an array (not a
 // temporary) of any element type.
 bool unit_stride_view(const bh_view &v, int axis, const Symbols &sym) {
@@ -1527,14 +1539,13 @@ void emit_flat_vector(Symbols &sym, ostream &body, const CodegenOptions &opt, co
     for (const bh_view &v : outs) align_check(v);
     body << "        }\n";
     Scope scope;
-    for (size_t k = 0; k < pre.size(); ++k) {
-        const string T = cuda_type(pre[k].base->dtype());
-        body << "        " << T << " pl" << k << "[4];\n";
-        const int bytes = 4 * static_cast<int>(bh_type_size(pre[k].base->dtype()));
-        if (vec_pre[k]) {
+    // The thread's 4 elements of view `v` into the register array `dst`.
+    auto emit_load = [&](const string &dst, const bh_view &v, bool words) {
+        const int bytes = 4 * static_cast<int>(bh_type_size(v.base->dtype()));
+        if (words) {
             body << "        if (vec) {\n";
             body << "            " << fi.decl("0") << "\n";
-            body << "            " << word_copy("pl" + to_string(k), "&" + em.array_ref(pre[k]), bytes) << "\n";
+            body << "            " << word_copy(dst, "&" + em.array_ref(v), bytes) << "\n";
             body << "        } else {\n";
         } else {
             body << "        {\n";
@@ -1542,13 +1553,18 @@ void emit_flat_vector(Symbols &sym, ostream &body, const CodegenOptions &opt, co
         body << "#pragma unroll\n";
         body << "            for (int j = 0; j < 4; ++j) {\n";
         body << "                " << fi.decl("j") << "\n";
-        body << "                pl" << k << "[j] = " << em.array_ref(pre[k]) << ";\n";
+        body << "                " << dst << "[j] = " << em.array_ref(v) << ";\n";
         body << "            }\n";
         body << "        }\n";
+    };
+    for (size_t k = 0; k < pre.size(); ++k) {
+        body << "        " << cuda_type(pre[k].base->dtype()) << " pl" << k << "[4];\n";
+        emit_load("pl" + to_string(k), pre[k], vec_pre[k]);
         scope.repl[ViewKey(pre[k])] = "pl" + to_string(k) + "[j]";
     }
     for (size_t k = 0; k < outs.size(); ++k) {
         body << "        " << cuda_type(outs[k].base->dtype()) << " so" << k << "[4];\n";
+        if (read_before_written(inner, outs[k])) emit_load("so" + to_string(k), outs[k], true);
         scope.repl[ViewKey(outs[k])] = "so" + to_string(k) + "[j]";
     }
     body << "#pragma unroll\n";
@@ -3078,7 +3094,7 @@ LaunchUnit lower_grid_reduce(const LoopB &loop, const vector<InstrPtr> &identiti
                 continue;
             const bh_view &v = i->operand[0];
             if (!unit_stride_view(v, 0, sym) || sym.always_array.count(v.base) || touched[v.base].size() != 1) continue;
-            if (acc_k.count(ViewKey(v))) continue;
+            if (acc_k.count(ViewKey(v)) || read_before_written(L, v)) continue;
             if (seen.insert(ViewKey(v)).second) wouts.push_back(v);
         }
     }
@@ -3416,6 +3432,45 @@ bool scan1d_applicable(const LoopB &loop, InstrPtr &acc) {
         if (!i->operand.empty() && !i->operand[0].isConstant() && i->operand[0].base == acc->operand[0].base)
             return false;
     }
+    return true;
+}
+
+// The instructions of a SCAN1D loop before its accumulate run once per unit: they may not update an
+// array in place. When some do and no temporary leaves them, `maps` receives the loop of those
+// instructions and `rest` the loop without them (two kernels in order); false when neither holds.
+bool split_in_place_updates(const LoopB &loop, const InstrPtr &acc, LoopB &maps, LoopB &rest, bool &split) {
+    set<const bh_base *> read, written, temps;
+    for (const bh_base *b : loop.getLocalTemps()) temps.insert(b);
+    split = false;
+    bool before = true, crosses = false;
+    maps = loop;
+    rest = loop;
+    maps._block_list.clear();
+    rest._block_list.clear();
+    for (const Block &b : loop._block_list) {
+        const InstrPtr &i = b.getInstr();
+        if (i == acc) before = false;
+        if (bh_opcode_is_system(i->opcode)) {
+            rest._block_list.push_back(b);
+            continue;
+        }
+        if (before) {
+            for (size_t o = 1; o < i->operand.size(); ++o)
+                if (!i->operand[o].isConstant() && !written.count(i->operand[o].base)) read.insert(i->operand[o].base);
+            written.insert(i->operand[0].base);
+            if (read.count(i->operand[0].base)) split = true;
+            maps._block_list.push_back(b);
+        } else {
+            for (size_t o = 1; o < i->operand.size(); ++o)
+                if (!i->operand[o].isConstant() && temps.count(i->operand[o].base) && written.count(i->operand[o].base))
+                    crosses = true;
+            rest._block_list.push_back(b);
+        }
+    }
+    if (!split) return true;
+    if (crosses) return false;
+    maps.metadataUpdate();
+    rest.metadataUpdate();
     return true;
 }
 
@@ -4836,12 +4891,17 @@ vector<LaunchUnit> lower_kernel(const LoopB &kernel, const CodegenOptions &opt) 
                 const bh_view &v = jitk::all_instr(*il)[0]->operand[0];
                 ok = ok && v.base == scan_acc->operand[0].base;
             }
+            LoopB maps, rest;
+            bool split = false;
+            ok = ok && split_in_place_updates(L, scan_acc, maps, rest, split);
             if (ok) {
                 pending_id_loops.clear();
+                if (split) units.push_back(lower_flat(maps, 1, opt));
+                const LoopB &S = split ? rest : L;
                 if (opt.scan_single_pass && !opt.bounds_check) {
-                    units.push_back(lower_scan1d_single(L, scan_acc, opt));
+                    units.push_back(lower_scan1d_single(S, scan_acc, opt));
                 } else {
-                    for (LaunchUnit &su : lower_scan1d(L, scan_acc, opt)) units.push_back(std::move(su));
+                    for (LaunchUnit &su : lower_scan1d(S, scan_acc, opt)) units.push_back(std::move(su));
                 }
                 continue;
             }

@@ -1809,8 +1809,15 @@ bool lower_tile2d(const LoopB &loop, const CodegenOptions &opt, LaunchUnit &u) {
     u.rows = L.size;
     u.cols = inner.size;
     const int64_t tiles_c = (u.cols + kTileCols - 1) / kTileCols;
-    ParamLayout pl;
+    // Rows or starts off the 16-byte boundary rule TMA out for every array of this shape: the unit
+    // then has no tensor maps and no ring, whose 64 KB would leave three CTAs on an SM.
+    bool tma = true;
     for (size_t k = 0; k < tv.size(); ++k) {
+        const int64_t ld = tpose[k] ? tv[k].stride[1] : tv[k].stride[0];
+        tma = tma && (ld * esize) % 16 == 0 && tv[k].start >= 0 && (tv[k].start % ld * esize) % 16 == 0;
+    }
+    ParamLayout pl;
+    for (size_t k = 0; tma && k < tv.size(); ++k) {
         // A transposed view's tile is TR elements along its base rows x 64 rows (128-byte swizzle);
         // a row-wise view's tile is 64 elements along its base rows x TR rows (no swizzle).
         ParamField f{ParamField::TMAP};
@@ -1827,23 +1834,25 @@ bool lower_tile2d(const LoopB &loop, const CodegenOptions &opt, LaunchUnit &u) {
     add_common_fields(sym, pl, opt);
     pl.add(work_field(tiles_c), "bh_i64", "tiles_c");
     pl.add(work_field(u.work_items()), "bh_i64", "work");
-    for (size_t k = 0; k < tv.size(); ++k) {
+    for (size_t k = 0; tma && k < tv.size(); ++k) {
         // Tensor coordinates of the view's element (0, 0): column and row of its base array.
         const int64_t ld = tpose[k] ? tv[k].stride[1] : tv[k].stride[0];
         pl.add(work_field(tv[k].start >= 0 ? tv[k].start % ld : 0), "bh_i64", "tx" + to_string(k));
         pl.add(work_field(tv[k].start >= 0 ? tv[k].start / ld : 0), "bh_i64", "ty" + to_string(k));
     }
-    ParamField ok{ParamField::TMA_OK};
-    pl.add(ok, "bh_i64", "tma_ok");
-    ParamField err{ParamField::SCRATCH};
-    err.i64 = -1;  // the engine's error record
-    pl.add(err, "unsigned long long*", "err");
-    pl.pad64();
+    if (tma) {
+        ParamField ok{ParamField::TMA_OK};
+        pl.add(ok, "bh_i64", "tma_ok");
+        ParamField err{ParamField::SCRATCH};
+        err.i64 = -1;  // the engine's error record
+        pl.add(err, "unsigned long long*", "err");
+        pl.pad64();
+    }
 
     const string T = cuda_type(tv[0].base->dtype());
     const string rows = "p.n" + to_string(sym.loop_id.at(&L)), cols = "p.n" + to_string(sym.loop_id.at(&inner));
     stringstream body;
-    body << "// bh_dynamic_shared_bytes: " << stages * static_cast<int>(tv.size()) * kTileBoxBytes + 1024 << "\n";
+    if (tma) body << "// bh_dynamic_shared_bytes: " << stages * static_cast<int>(tv.size()) * kTileBoxBytes + 1024 << "\n";
     body << "template <bool STAGED> __device__ __forceinline__ void bh_tile(const P &p, bh_i64 w, const unsigned char *stage) {\n";
     body << pointer_locals(sym);
     body << "    const bh_i64 tr = w / p.tiles_c;\n";
@@ -1867,6 +1876,50 @@ bool lower_tile2d(const LoopB &loop, const CodegenOptions &opt, LaunchUnit &u) {
         body << "        memcpy((char *)&tv" << k << "[0] + 16, &q1, 16);\n";
         body << "    }\n";
     }
+    // Without TMA the boxes go through shared memory all the same: neighbouring threads load
+    // neighbouring elements of a base row (TR of them), all loads of the tile before the barrier.
+    {
+        Emitter es(sym, body, opt);
+        body << "    if (!STAGED) {\n";
+        for (size_t k = 0; k < tv.size(); ++k) {
+            body << "        " << T << " ld" << k << "[" << RPT << "];\n";
+            if (tpose[k]) body << "        __shared__ " << T << " box" << k << "[" << kTileCols * (TR + 1) << "];\n";
+        }
+        body << "#pragma unroll\n";
+        body << "        for (int e = 0; e < " << RPT << "; ++e) {\n";
+        for (size_t k = 0; k < tv.size(); ++k) {
+            body << "            {\n";
+            if (tpose[k]) {
+                body << "                const int at = e * " << kThreads << " + threadIdx.x;\n";
+                body << "                const bh_i64 i0 = tr * " << TR << " + at % " << TR << ", i1 = tc * 64 + at / " << TR << ";\n";
+            } else {
+                body << "                const bh_i64 i0 = rbase + e;\n";
+            }
+            body << "                if (i0 < " << rows << " && i1 < " << cols << ") ld" << k << "[e] = " << es.array_ref(tv[k]) << ";\n";
+            body << "            }\n";
+        }
+        body << "        }\n";
+        body << "        __syncthreads();\n";  // the previous tile's boxes have been read
+        body << "#pragma unroll\n";
+        body << "        for (int e = 0; e < " << RPT << "; ++e) {\n";
+        body << "            const int at = e * " << kThreads << " + threadIdx.x;\n";
+        body << "            (void)at;\n";
+        for (size_t k = 0; k < tv.size(); ++k) {
+            if (tpose[k]) {
+                body << "            box" << k << "[at / " << TR << " * " << TR + 1 << " + at % " << TR << "] = ld" << k << "[e];\n";
+            } else {
+                body << "            tv" << k << "[e] = ld" << k << "[e];\n";
+            }
+        }
+        body << "        }\n";
+        body << "        __syncthreads();\n";
+        body << "#pragma unroll\n";
+        body << "        for (int e = 0; e < " << RPT << "; ++e) {\n";
+        for (size_t k = 0; k < tv.size(); ++k)
+            if (tpose[k]) body << "            tv" << k << "[e] = box" << k << "[c * " << TR + 1 << " + rq * " << RPT << " + e];\n";
+        body << "        }\n";
+        body << "    }\n";
+    }
     for (int path = 0; path < 2; ++path) {
         body << (path == 0 ? "    if (rbase + " + to_string(RPT) + " <= " + rows + " && i1 < " + cols + ") {\n"
                            : "    } else {\n");
@@ -1878,11 +1931,7 @@ bool lower_tile2d(const LoopB &loop, const CodegenOptions &opt, LaunchUnit &u) {
         body << "            const bh_i64 i0 = rbase + e;\n";
         if (path == 1) body << "            if (i0 >= " << rows << " || i1 >= " << cols << ") break;\n";
         for (size_t k = 0; k < tv.size(); ++k) {
-            if (tpose[k]) {
-                body << "            if (!STAGED) tv" << k << "[e] = " << eb.array_ref(tv[k]) << ";\n";
-            } else {
-                body << "            tv" << k << "[e] = STAGED ? tr" << k << "[e * 64] : " << eb.array_ref(tv[k]) << ";\n";
-            }
+            if (!tpose[k]) body << "            if (STAGED) tv" << k << "[e] = tr" << k << "[e * 64];\n";
         }
         declare_chain_temps(eb, sym, scope, chain, 1, body, 12);
         eb.write_body(inner, scope, 12);
@@ -1890,6 +1939,14 @@ bool lower_tile2d(const LoopB &loop, const CodegenOptions &opt, LaunchUnit &u) {
     }
     body << "    }\n}\n";
     body << "__device__ __forceinline__ void bh_work(const P &p, bh_i64 w) { bh_tile<false>(p, w, nullptr); }\n";
+    if (!tma) {
+        body << kWrappers;
+        u.fields = pl.fields;
+        u.algorithmic_bytes = unit_bytes(sym, vector<const Block *>{&holder});
+        u.elements = u.rows * u.cols;
+        finish_source(u, pl.decl.str(), body.str(), opt);
+        return true;
+    }
     // One thread issues a tile's boxes: expect their bytes on the stage's barrier, then copy.
     body << "__device__ __forceinline__ void bh_tile_issue(const P &p, bh_i64 w, unsigned char *stage, unsigned long long *bar) {\n";
     body << "    const bh_i64 tr = w / p.tiles_c;\n";

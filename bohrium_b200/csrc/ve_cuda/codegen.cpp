@@ -6,6 +6,7 @@
 // reduction outputs follow core/jitk/engines/engine.cpp:84-249.
 #include <algorithm>
 #include <cassert>
+#include <cmath>
 #include <cstring>
 #include <functional>
 #include <map>
@@ -36,6 +37,26 @@ const char *sched_name(Sched s) {
         case Sched::TILE2D: return "tile2d";
     }
     return "?";
+}
+
+namespace {
+template <typename T> T exact_reciprocal(T c) {
+    int e = 0;
+    if (!isfinite(c) || fabs(frexp(c, &e)) != static_cast<T>(0.5)) return 0;
+    const T r = static_cast<T>(1) / c;
+    return isnormal(r) && isnormal(c) ? r : static_cast<T>(0);
+}
+} // namespace
+
+double power_of_two_reciprocal(const bh_constant &c) {
+    if (c.type == bh_type::FLOAT32) return exact_reciprocal(c.value.float32);
+    if (c.type == bh_type::FLOAT64) return exact_reciprocal(c.value.float64);
+    return 0;
+}
+
+bool divides_by_power_of_two(const bh_instruction &i) {
+    return i.opcode == BH_DIVIDE && i.operand.size() == 3 && !i.operand[1].isConstant() && i.operand[2].isConstant() &&
+           i.operand[0].base->dtype() == i.constant.type && power_of_two_reciprocal(i.constant) != 0;
 }
 
 int64_t LaunchUnit::work_items() const {
@@ -132,18 +153,36 @@ __device__ __forceinline__ void bh_grid_dependency() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-__device__ __forceinline__ bh_u64 bh_random123(bh_u64 start, bh_u64 key, bh_u64 index) {
+// 0, but a value of each thread for the compiler: a key plus this one keeps its round keys in
+// registers, shared by the elements of a thread. From the kernel's parameter they were added up
+// again for every element on the uniform pipe, a quarter of the generator's instructions.
+__device__ __forceinline__ unsigned bh_thread_zero() {
+    unsigned lane;
+    asm("mov.u32 %0, %%laneid;" : "=r"(lane));
+    return __umulhi(lane, 1u << 27);
+}
+
+__device__ __forceinline__ bh_u64 bh_random123(bh_u64 start, unsigned key, bh_u64 index) {
     const bh_u64 c = start + index;
-    unsigned x0 = (unsigned)c, x1 = (unsigned)(c >> 32), k = (unsigned)key;
+    unsigned x0 = (unsigned)c, x1 = (unsigned)(c >> 32), k = key;
 #pragma unroll
     for (int r = 0; r < 10; ++r) {
-        const unsigned hi = __umulhi(0xD256D193u, x0);
-        const unsigned lo = 0xD256D193u * x0;
-        x0 = hi ^ k ^ x1;
-        x1 = lo;
+        // one 32 x 32 -> 64 bit product: separate high and low multiplies take two
+        const bh_u64 m = (bh_u64)0xD256D193u * x0;
+        x0 = (unsigned)(m >> 32) ^ k ^ x1;
+        x1 = (unsigned)m;
         k += 0x9E3779B9u;
     }
     return ((bh_u64)x1 << 32) | (bh_u64)x0;
+}
+
+// The nearest double to an unsigned 64-bit integer (ties to even), as the conversion gives: the
+// halves become 2^84 + hi 2^32 and 2^52 + lo by their bits, the first difference is exact, and the
+// sum rounds once.
+__device__ __forceinline__ double bh_u64_to_double(bh_u64 v) {
+    const double hi = __hiloint2double(0x45300000, (int)(unsigned)(v >> 32));
+    const double lo = __hiloint2double(0x43300000, (int)(unsigned)v);
+    return (hi - 19342813118337666422669312.0) + lo;
 }
 
 template <typename T> __device__ __forceinline__ T bh_shfl_xor(T v, int m) {
@@ -912,7 +951,7 @@ public:
         } else if (instr.opcode == BH_RANDOM) {
             ops.push_back(name(instr.operand[0], s));
             const int cid = sym.const_id.at(&instr);
-            ops.push_back("bh_random123(p.c" + to_string(cid) + "_start, p.c" + to_string(cid) + "_key, (bh_u64)" +
+            ops.push_back("bh_random123(p.c" + to_string(cid) + "_start, rk" + to_string(cid) + ", (bh_u64)" +
                           index_expr(instr.operand[0]) + ")");
         } else if (instr.opcode == BH_GATHER) {
             ops.push_back(name(instr.operand[0], s));
@@ -952,6 +991,16 @@ public:
             }
         }
         indent(ind);
+        if (divides_by_power_of_two(instr)) {
+            // the product is the correctly rounded quotient, bit for bit
+            out << ops[0] << " = " << ops[1] << " * " << ops[2] << "_r;\n";
+            return;
+        }
+        if (instr.opcode == BH_IDENTITY && !instr.operand[1].isConstant() && instr.operand[0].base->dtype() == bh_type::FLOAT64 &&
+            instr.operand[1].base->dtype() == bh_type::UINT64) {
+            out << ops[0] << " = bh_u64_to_double(" << ops[1] << ");\n";
+            return;
+        }
         out << op_statement(instr, ops) << "\n";
     }
 
@@ -1086,6 +1135,10 @@ void add_common_fields(Symbols &sym, ParamLayout &pl, const CodegenOptions &opt)
             f.c = instr->constant;
             f.origin = instr->origin_id;
             pl.add(f, cuda_type(instr->constant.type), "c" + to_string(i));
+            if (divides_by_power_of_two(*instr)) {
+                f.kind = ParamField::RECIPROCAL;
+                pl.add(f, cuda_type(instr->constant.type), "c" + to_string(i) + "_r");
+            }
         }
     }
     if (opt.bounds_check) {
@@ -1195,11 +1248,14 @@ void finish_source(LaunchUnit &u, const string &params_decl, const string &body,
     u.source = s;
 }
 
-// Unpack the pointer fields into local restrict pointers.
+// Unpack the pointer fields into local restrict pointers, and the generators' keys into registers.
 string pointer_locals(const Symbols &sym) {
     stringstream ss;
     for (size_t i = 0; i < sym.params.size(); ++i)
         ss << "    " << cuda_type(sym.params[i]->dtype()) << "* __restrict__ a" << i << " = p.a" << i << ";\n";
+    for (size_t i = 0; i < sym.consts.size(); ++i)
+        if (sym.consts[i]->constant.type == bh_type::R123)
+            ss << "    const unsigned rk" << i << " = (unsigned)p.c" << i << "_key + bh_thread_zero();\n";
     return ss.str();
 }
 

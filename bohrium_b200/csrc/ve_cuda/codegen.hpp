@@ -81,6 +81,14 @@ int contract_multiply_add(std::vector<bh_instruction> &list, const std::set<bh_b
                           const std::function<bool(const bh_base *)> &holds_nothing = nullptr);
 const char *sched_name(Sched s);
 
+// 1 / c for a float32 or float64 constant that is a power of two, both it and its reciprocal normal
+// numbers; else 0.
+double power_of_two_reciprocal(const bh_constant &c);
+// `x / c` with such a constant: written as x * (1 / c), the same number bit for bit (an IEEE division
+// takes some ten instructions and a branch per element). It is a property of the constant's value, so
+// it is part of a flush's structure: plans are not shared between divisors of the two kinds.
+bool divides_by_power_of_two(const bh_instruction &i);
+
 constexpr int kThreads = 256;      // threads per CTA for every schedule
 constexpr int kReduceV = 8;        // elements per thread per tile in GRID_REDUCE
 constexpr int64_t kReduceTile = kThreads * kReduceV;
@@ -89,10 +97,11 @@ constexpr int64_t kScanChunk = 4096; // elements per chunk in SCAN1D
 
 // One 8-byte slot (or two for 16-byte constants) of the kernel parameter struct.
 struct ParamField {
-    enum Kind { PTR, I64, CONST, R123_START, R123_KEY, SCRATCH, COUNTER, TMAP, TMA_OK } kind;
+    enum Kind { PTR, I64, CONST, RECIPROCAL, R123_START, R123_KEY, SCRATCH, COUNTER, TMAP, TMA_OK } kind;
     bh_base *base = nullptr; // PTR
     int64_t i64 = 0;         // I64
-    bh_constant c{};         // CONST / R123_*
+    bh_constant c{};         // CONST / RECIPROCAL / R123_*
+    // RECIPROCAL: 1 / constant, a divisor that is a power of two (divides_by_power_of_two).
     int64_t origin = -1;     // CONST / R123_*: origin id of the instruction holding the constant
     int part = 0;            // CONST: which 8 bytes of the constant (1: the imaginary part of a complex128)
     int64_t off = 0;         // COUNTER: index offset in the unit's counters

@@ -801,6 +801,18 @@ void EngineCUDA::pack_params(const PlanUnit &pu, const vector<bh_base *> &bases,
                        static_cast<size_t>(min<int64_t>(bh_type_size(f.c.type), 8)));
                 break;
             }
+            case ParamField::RECIPROCAL: {
+                const bh_constant &c =
+                    f.origin >= 0 && f.origin < static_cast<int64_t>(instrs.size()) ? instrs[f.origin]->constant : f.c;
+                const double r = power_of_two_reciprocal(c);
+                const float rf = static_cast<float>(r);
+                if (f.c.type == bh_type::FLOAT32) {
+                    memcpy(slot, &rf, sizeof(rf));
+                } else {
+                    memcpy(slot, &r, sizeof(r));
+                }
+                break;
+            }
             case ParamField::R123_START:
             case ParamField::R123_KEY: {
                 const bh_constant &c =
@@ -1097,7 +1109,7 @@ uint64_t hash_instr_list(const vector<bh_instruction *> &instr_list, vector<bh_b
     for (const bh_instruction *instr : instr_list) {
         h.add(static_cast<uint64_t>(instr->opcode));
         h.add(static_cast<uint64_t>(instr->sweep_axis()));
-        h.add(instr->constructor ? 1 : 0);
+        h.add((instr->constructor ? 1 : 0) | (divides_by_power_of_two(*instr) ? 2 : 0));
         for (const bh_view &v : instr->operand) {
             if (v.isConstant()) {
                 h.add(0xC0115747ULL);
@@ -1239,7 +1251,7 @@ uint64_t EngineCUDA::prepare(vector<bh_instruction> &list, vector<bh_instruction
                 h.add(static_cast<uint64_t>(v.stride[d]));
             }
         }
-        h.add(instr.constructor ? 1 : 0);
+        h.add((instr.constructor ? 1 : 0) | (divides_by_power_of_two(instr) ? 2 : 0));
         out.push_back(&instr);
     }
     h.add(out.size());

@@ -3109,7 +3109,7 @@ LaunchUnit lower_grid_reduce(const LoopB &loop, const vector<InstrPtr> &identiti
         both << "__device__ __forceinline__ void bh_work(const P &p, bh_i64 w) { bh_kp::bh_work(p, w); }\n";
         both << "__device__ __forceinline__ void bh_batch_work(const P &p, bh_i64 w) { bh_kg::bh_work(p, w); }\n";
         if (up.tail_capable) both << "__device__ __forceinline__ void bh_tail(const P &p) { bh_kp::bh_tail(p); }\n";
-        both << kMainWrapper << kKernels;
+        both << "__device__ __forceinline__ void bh_main(const P &p) { bh_kp::bh_main(p); }\n" << kKernels;
         LaunchUnit u2 = up;
         u2.batch_chunks = Kg;
         finish_source(u2, up.params_decl, both.str(), opt);
@@ -3157,15 +3157,15 @@ LaunchUnit lower_grid_reduce(const LoopB &loop, const vector<InstrPtr> &identiti
         helpers << block_reduce_all_fn(ctypes, ops, idents, offsets, K);
     }
     body << helpers.str();
-    body << "__device__ void bh_work(const P &p, bh_i64 w) {\n";
-    body << pointer_locals(sym);
-    body << "    __shared__ alignas(16) unsigned long long sm_raw[" << (sm_bytes + 7) / 8 << "];\n";
-    body << "    __shared__ bool am_last;\n";
-    for (size_t k = 0; k < reds.size(); ++k)
-        body << "    " << ctypes[k] << "* part" << k << " = (" << ctypes[k] << "*)(p.scratch + p.ntiles * "
-             << u.slot_bytes * k << ");\n";
+    // bh_fold: the K tiles of work item w folded by this thread into its accumulators.
+    string acc_params, acc_args;
     for (size_t k = 0; k < reds.size(); ++k) {
-        body << "    " << ctypes[k] << " " << accs[k] << "[" << K << "];\n";
+        acc_params += ", " + ctypes[k] + " (&" + accs[k] + ")[" + KT + "]";
+        acc_args += ", " + accs[k];
+    }
+    body << "__device__ __forceinline__ void bh_fold(const P &p, bh_i64 w" << acc_params << ") {\n";
+    body << pointer_locals(sym);
+    for (size_t k = 0; k < reds.size(); ++k) {
         body << "#pragma unroll\n";
         body << "    for (int k = 0; k < " << K << "; ++k) " << accs[k] << "[k] = " << idents[k] << ";\n";
     }
@@ -3309,6 +3309,48 @@ LaunchUnit lower_grid_reduce(const LoopB &loop, const vector<InstrPtr> &identiti
         if (vectorized)
             for (size_t m = 0; m < wouts.size(); ++m) scope.repl[ViewKey(wouts[m])] = "so" + to_string(m) + "[j]";
     };
+    // A full tile of a heavy body in two halves of 4 elements: the half's inputs, its elements, its
+    // written words, then the other half by the same code. Half the registers for inputs (one
+    // Black-Scholes flush of 10M options: 60 instead of 78, 4 CTAs on an SM instead of 3) and half
+    // the code: 166 instead of 188 us; halves of the halves took 168 us.
+    auto emit_half_tiles = [&](Emitter &eb) {
+        body << "        const int k = 0;\n";
+        body << "#pragma unroll 1\n";
+        body << "        for (int g = 0; g < 2; ++g) {\n";
+        body << "            const bh_i64 ib = tile0 * " << kReduceTile << " + g * " << kReduceTile / 2 << " + threadIdx.x * 4;\n";
+        auto move = [&](const bh_view &v, const string &reg, bool load, bool words) {
+            const int bytes = 4 * static_cast<int>(bh_type_size(v.base->dtype()));
+            const string ref = eb.array_ref(v);
+            if (words) {
+                body << "            if (vec) { const bh_i64 i0 = ib; "
+                     << (load ? word_copy(reg, "&" + ref, bytes) : word_copy("&" + ref, reg, bytes)) << "} else {\n";
+            } else {
+                body << "            {\n";
+            }
+            body << "#pragma unroll\n";
+            body << "                for (int j = 0; j < 4; ++j) { const bh_i64 i0 = ib + j; "
+                 << (load ? reg + "[j] = " + ref : ref + " = " + reg + "[j]") << "; }\n";
+            body << "            }\n";
+        };
+        Scope half;
+        for (size_t v = 0; v < pre.size(); ++v) {
+            const string reg = "pl" + to_string(v);
+            body << "            " << cuda_type(pre[v].base->dtype()) << " " << reg << "[4];\n";
+            move(pre[v], reg, true, vec_pre[v]);
+            half.repl[ViewKey(pre[v])] = reg + "[j]";
+        }
+        for (size_t m = 0; m < wouts.size(); ++m) {
+            body << "            " << cuda_type(wouts[m].base->dtype()) << " so" << m << "[4];\n";
+            half.repl[ViewKey(wouts[m])] = "so" + to_string(m) + "[j]";
+        }
+        body << "#pragma unroll\n";
+        body << "            for (int j = 0; j < 4; ++j) {\n";
+        body << "                const bh_i64 i0 = ib + j;\n";
+        eb.write_body(L, half, 16);
+        body << "            }\n";
+        for (size_t m = 0; m < wouts.size(); ++m) move(wouts[m], "so" + to_string(m), false, true);
+        body << "        }\n";
+    };
     // Path 0: all K tiles of the item are full. Every input of all K x 8 elements of the thread is
     // loaded first, then the tiles are computed.
     {
@@ -3317,6 +3359,9 @@ LaunchUnit lower_grid_reduce(const LoopB &loop, const vector<InstrPtr> &identiti
         Emitter eb(sym, body, opt);
         eb.external_acc = acc_k;
         if (vectorized) emit_vec_check(eb);
+        if (heavy && vectorized && K == 1) {
+            emit_half_tiles(eb);
+        } else {
         if (!pre.empty()) {
             emit_pl_decls();
             body << "#pragma unroll\n";
@@ -3345,6 +3390,7 @@ LaunchUnit lower_grid_reduce(const LoopB &loop, const vector<InstrPtr> &identiti
             emit_full_tile(eb, scope, 12);
         }
         body << "        }\n";
+            }
     }
     // Path 1: the last work item. Its full tiles (kfull of them) take the same code as path 0,
     // one tile at a time; the partial tile checks every index. Both fold elements j = 0..7 of
@@ -3380,7 +3426,54 @@ LaunchUnit lower_grid_reduce(const LoopB &loop, const vector<InstrPtr> &identiti
         body << string(static_cast<size_t>(ind), ' ') << "}\n";
         body << "        }\n";
     }
-    body << "    }\n";
+    body << "    }\n}\n";
+    auto emit_partials = [&]() {
+        for (size_t k = 0; k < reds.size(); ++k)
+            body << "    " << ctypes[k] << "* part" << k << " = (" << ctypes[k] << "*)(p.scratch + p.ntiles * "
+                 << u.slot_bytes * k << ");\n";
+    };
+    // The CTA that arrives last folds the tile partials: thread t those of tiles t, t + 256, ... in
+    // order (eight loads in flight), then one block tree.
+    auto emit_last = [&]() {
+        body << "    bh_acquire();\n";
+        for (size_t k = 0; k < reds.size(); ++k) {
+            const InstrPtr &r = reds[k];
+            body << "    {\n";
+            body << "        " << ctypes[k] << " acc = " << idents[k] << ";\n";
+            body << "        bh_i64 t = threadIdx.x;\n";
+            body << "        for (; t + " << 7 * kThreads << " < p.ntiles; t += " << 8 * kThreads << ") {\n";
+            body << "            " << ctypes[k] << " x[8];\n";
+            body << "#pragma unroll\n";
+            body << "            for (int j = 0; j < 8; ++j) x[j] = bh_ldcg(part" << k << " + t + j * " << kThreads << ");\n";
+            body << "#pragma unroll\n";
+            body << "            for (int j = 0; j < 8; ++j) acc = " << reduce_expr(r->opcode, "acc", "x[j]") << ";\n";
+            body << "        }\n";
+            body << "        for (; t < p.ntiles; t += " << kThreads << ") {\n";
+            body << "            const " << ctypes[k] << " x = bh_ldcg(part" << k << " + t);\n";
+            body << "            acc = " << reduce_expr(r->opcode, "acc", "x") << ";\n";
+            body << "        }\n";
+            body << "        acc = bh_block_reduce" << k << "(acc, (" << ctypes[k] << "*)sm_raw);\n";
+            if (!sym.temps.count(r->operand[0].base)) {
+                body << "        if (threadIdx.x == 0) " << em.array_ref(r->operand[0]) << " = acc;\n";
+            }
+            body << "    }\n";
+        }
+        body << "    if (threadIdx.x == 0) *p.counter = 0u;\n";
+    };
+    auto emit_accs = [&](int ind) {
+        for (size_t k = 0; k < reds.size(); ++k)
+            body << string(static_cast<size_t>(ind), ' ') << ctypes[k] << " " << accs[k] << "[" << K << "];\n";
+    };
+    // A work item of a grouped launch: its tiles' block trees and its arrival, one item at a time.
+    body << "__device__ void bh_work(const P &p, bh_i64 w) {\n";
+    body << pointer_locals(sym);
+    body << "    __shared__ alignas(16) unsigned long long sm_raw[" << (sm_bytes + 7) / 8 << "];\n";
+    body << "    __shared__ bool am_last;\n";
+    emit_partials();
+    emit_accs(4);
+    body << "    const bh_i64 tile0 = w * " << KT << ";\n";
+    body << "    const int ktiles = (int)min((bh_i64)" << KT << ", p.ntiles - tile0);\n";
+    body << "    bh_fold(p, w" << acc_args << ");\n";
     if (reds.size() > 1) {
         body << "    bh_block_reduce_all(";
         for (size_t k = 0; k < reds.size(); ++k) body << accs[k] << ", ";
@@ -3400,22 +3493,80 @@ LaunchUnit lower_grid_reduce(const LoopB &loop, const vector<InstrPtr> &identiti
     body << "    }\n";
     body << "    __syncthreads();\n";
     body << "    if (!am_last) return;\n";
-    body << "    bh_acquire();\n";
+    emit_last();
+    body << "}\n";
+    // A plain launch: the CTA folds all its items before it arrives once. The warps' trees of up to
+    // `held` tiles are kept in shared memory, and one thread per tile finishes the block tree in the
+    // order of bh_block_reduce (lanes 8..31 there hold the identity), so no tile waits at a barrier
+    // or for an atomic's round trip (one of each per tile before: pi from 5e7 random points 231 us, now
+    // 203; the plain chain of 2^20 float64 17.2 and 15.4 us).
+    int64_t warp_bytes = 0;
+    vector<int64_t> warp_off;
     for (size_t k = 0; k < reds.size(); ++k) {
-        const InstrPtr &r = reds[k];
-        body << "    {\n";
-        body << "        " << ctypes[k] << " acc = " << idents[k] << ";\n";
-        body << "        for (bh_i64 t = threadIdx.x; t < p.ntiles; t += " << kThreads << ") {\n";
-        body << "            const " << ctypes[k] << " x = bh_ldcg(part" << k << " + t);\n";
-        body << "            acc = " << reduce_expr(r->opcode, "acc", "x") << ";\n";
-        body << "        }\n";
-        body << "        acc = bh_block_reduce" << k << "(acc, (" << ctypes[k] << "*)sm_raw);\n";
-        if (!sym.temps.count(r->operand[0].base)) {
-            body << "        if (threadIdx.x == 0) " << em.array_ref(r->operand[0]) << " = acc;\n";
-        }
-        body << "    }\n";
+        warp_off.push_back(warp_bytes);
+        warp_bytes += (kThreads / 32) * bh_type_size(reds[k]->operand[0].base->dtype());
     }
-    body << "    if (threadIdx.x == 0) *p.counter = 0u;\n";
+    const int64_t held = max<int64_t>(K, min<int64_t>(64, 8192 / warp_bytes) / K * K);
+    body << "__device__ __forceinline__ void bh_main(const P &p) {\n";
+    body << pointer_locals(sym);
+    body << "    __shared__ alignas(16) unsigned long long sm_raw[" << (sm_bytes + 7) / 8 << "];\n";
+    body << "    __shared__ alignas(16) unsigned char warp_sm[" << (held * warp_bytes + 15) / 16 * 16 << "];\n";
+    body << "    __shared__ bool am_last;\n";
+    emit_partials();
+    for (size_t k = 0; k < reds.size(); ++k)
+        body << "    " << ctypes[k] << "* ws" << k << " = (" << ctypes[k] << "*)(warp_sm + " << held * warp_off[k] << ");\n";
+    body << "    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;\n";
+    body << "    int held = 0;\n";
+    body << "    for (bh_i64 w = blockIdx.x; w < p.work; w += gridDim.x) {\n";
+    emit_accs(8);
+    body << "        bh_fold(p, w" << acc_args << ");\n";
+    for (size_t k = 0; k < reds.size(); ++k) {
+        body << "#pragma unroll\n";
+        body << "        for (int k = 0; k < " << K << "; ++k) {\n";
+        body << "#pragma unroll\n";
+        body << "            for (int m = 16; m >= 1; m >>= 1) { const " << ctypes[k] << " o = bh_shfl_xor(" << accs[k]
+             << "[k], m); " << accs[k] << "[k] = " << reduce_expr(reds[k]->opcode, accs[k] + "[k]", "o") << "; }\n";
+        body << "            if (lane == 0) ws" << k << "[(held + k) * " << kThreads / 32 << " + warp] = " << accs[k] << "[k];\n";
+        body << "        }\n";
+    }
+    body << "        held += " << K << ";\n";
+    body << "        if (held < " << held << " && w + gridDim.x < p.work) continue;\n";
+    body << "        __syncthreads();\n";
+    body << "        const int s = threadIdx.x;\n";
+    body << "        const bh_i64 tile = (w - (bh_i64)((held - 1 - s) / " << K << ") * gridDim.x) * " << K << " + s % " << K << ";\n";
+    body << "        if (s < held && tile < p.ntiles) {\n";
+    for (size_t k = 0; k < reds.size(); ++k) {
+        const bh_opcode op = reds[k]->opcode;
+        body << "            {\n";
+        body << "                " << ctypes[k] << " v[" << kThreads / 32 << "];\n";
+        body << "#pragma unroll\n";
+        body << "                for (int j = 0; j < " << kThreads / 32 << "; ++j) {\n";
+        body << "                    v[j] = ws" << k << "[s * " << kThreads / 32 << " + j];\n";
+        body << "                    const " << ctypes[k] << " o = " << idents[k] << ";\n";
+        body << "                    v[j] = " << reduce_expr(op, "v[j]", "o") << ";\n";
+        body << "                    v[j] = " << reduce_expr(op, "v[j]", "o") << ";\n";
+        body << "                }\n";
+        body << "#pragma unroll\n";
+        body << "                for (int m = " << kThreads / 64 << "; m >= 1; m >>= 1)\n";
+        body << "#pragma unroll\n";
+        body << "                    for (int j = 0; j < m; ++j) v[j] = " << reduce_expr(op, "v[j]", "v[j + m]") << ";\n";
+        body << "                part" << k << "[tile] = v[0];\n";
+        body << "            }\n";
+    }
+    body << "        }\n";
+    body << "        __syncthreads();\n";
+    body << "        held = 0;\n";
+    body << "    }\n";
+    body << "    if (threadIdx.x == 0) {\n";
+    body << "        // the CTA's items, all of K tiles but perhaps the last item of all\n";
+    body << "        const bh_i64 items = blockIdx.x < p.work ? (p.work - 1 - blockIdx.x) / gridDim.x + 1 : 0;\n";
+    body << "        const bool has_last = items > 0 && (p.work - 1) % gridDim.x == blockIdx.x;\n";
+    body << "        const unsigned mine = (unsigned)(items * " << K << " - (has_last ? p.work * " << K << " - p.ntiles : 0));\n";
+    body << "        am_last = mine > 0 && bh_arrive_n((unsigned*)p.counter, mine) + mine == (unsigned)p.ntiles;\n";
+    body << "    }\n";
+    body << "    __syncthreads();\n";
+    body << "    if (!am_last) return;\n";
+    emit_last();
     body << "}\n";
     // The whole reduction in one CTA, for another kernel's tail (fuse_tails): only for small
     // arrays and order-free reductions, where the fold order does not change the result.
@@ -3456,7 +3607,7 @@ LaunchUnit lower_grid_reduce(const LoopB &loop, const vector<InstrPtr> &identiti
         }
         body << "}\n";
     }
-    body << kWrappers;
+    body << kBatchWork << kKernels;
     u.fields = pl.fields;
     u.algorithmic_bytes = unit_bytes(sym, vector<const Block *>{&holder});
     u.elements = L.size;

@@ -33,6 +33,7 @@ const char *sched_name(Sched s) {
         case Sched::OUTER_REDUCE: return "outer_reduce";
         case Sched::SCAN1D: return "scan1d";
         case Sched::AXIS_SCAN: return "axis_scan";
+        case Sched::ROWS: return "rows";
         case Sched::SERIAL: return "serial";
         case Sched::TILE2D: return "tile2d";
     }
@@ -70,6 +71,7 @@ int64_t LaunchUnit::work_items() const {
             return (tiles + chunks - 1) / chunks;  // chunks: tiles per work item
         }
         case Sched::SPLIT_REDUCE: return (rows * cols + V - 1) / V * chunks;  // V: points per CTA
+        case Sched::ROWS:
         case Sched::LANE_REDUCE: {
             const int64_t per = kThreads / chunks;
             return (rows * cols + per - 1) / per;
@@ -5097,6 +5099,445 @@ LaunchUnit fuse_tail(const LaunchUnit &u1, const LaunchUnit &u2) {
     return u;
 }
 
+// --------------------------------------------------------------------------------------- ROWS
+// Row fusion: neighbouring kernels of a flush that work through the rows of the same index space
+// (reductions over the contiguous axis and maps, as a row-wise softmax or normalisation makes) run
+// as one kernel when every array that one of them writes is touched by the others in the same row
+// only. C lanes of a CTA hold a row in registers: each input is read once, what one stage writes is
+// read by the next from registers, reduction results are shared among the row's lanes, and arrays
+// that the flush creates and frees within the group never reach memory. The lanes fold and combine
+// as LANE_REDUCE's do (lane l takes elements l, l + C, ... and a shuffle tree combines the lanes).
+// A softmax over 20000 rows of 1500 float32 moved 600 MB in three kernels and 147 us; as one kernel
+// it moves 240 MB and takes 68 us (37 us at the measured copy rate); 20000 x 100 40 and 14 us, 200 x
+// 1500 18 and 10 us. Bound by the latency of the rows' chains (loads, shuffles, divisions) and by the
+// code, which is unrolled over a lane's elements: 12 elements a lane (64 lanes fewer to a row) took 103
+// us there and 24 took 232, so rows get lanes until each holds few elements.
+constexpr int64_t kRowElements = 6;      // elements of a row per lane aimed at
+constexpr int64_t kRowElementsMost = 12; // and at most (with a whole CTA on a row)
+constexpr int kRowRegisters = 48;        // 4-byte registers of a row that a lane may carry between stages
+
+struct RowStage {
+    const LoopB *loop = nullptr; // the rank-0 loop
+    const LoopB *sub = nullptr;  // the loop over the row
+    bool reduce = false;
+};
+
+// The stage a kernel would be, from its lowering: one LANE_REDUCE with one point axis (without staged
+// stencil rows), or one 2-D map.
+bool row_stage(const LoopB &kernel, const vector<LaunchUnit> &units, RowStage &st) {
+    if (units.size() != 1 || units[0].tail || units[0].source.find("bh_stage_row") != string::npos) return false;
+    if (units[0].sched != Sched::LANE_REDUCE && units[0].sched != Sched::FLAT) return false;
+    for (const Block &b : kernel._block_list) {
+        if (b.isSystemOnly()) continue;
+        if (b.isInstr() || st.loop != nullptr) return false;
+        st.loop = &b.getLoop();
+    }
+    if (st.loop == nullptr) return false;
+    const unsigned P = static_cast<unsigned>(jitk::parallel_ranks(*st.loop, 64).first);
+    if (units[0].sched == Sched::LANE_REDUCE) {
+        if (P != 1) return false;
+        st.sub = split_candidate(*st.loop);
+        st.reduce = true;
+        return st.sub != nullptr;
+    }
+    const vector<const LoopB *> chain = jitk::get_first_loop_blocks(*st.loop);
+    if (P != 2 || chain.size() != 2 || !chain[1]->isInnermost() || !chain[1]->_sweeps.empty()) return false;
+    int loops = 0;
+    for (const Block &b : st.loop->_block_list) {
+        if (b.isInstr() && !bh_opcode_is_system(b.getInstr()->opcode)) return false;
+        if (!b.isInstr() && !b.isSystemOnly()) ++loops;
+    }
+    st.sub = chain[1];
+    return loops == 1;
+}
+
+// Lowers `stages` (the kernels' loops, in order) as one unit; false when they are not row-local or
+// too large. `dropped`: arrays that nothing outside the group sees.
+bool lower_rows(const vector<RowStage> &stages, const set<const bh_base *> &dropped, const CodegenOptions &opt, LaunchUnit &u) {
+    const int64_t points = stages[0].loop->size, len = stages[0].sub->size;
+    vector<Block> holders;
+    holders.reserve(stages.size());
+    for (const RowStage &s : stages) holders.emplace_back(*s.loop);
+    vector<RowStage> st;
+    vector<const Block *> items;
+    set<const bh_instruction *> folded;
+    for (size_t i = 0; i < stages.size(); ++i) {
+        items.push_back(&holders[i]);
+        RowStage s;
+        s.loop = &holders[i].getLoop();
+        s.reduce = stages[i].reduce;
+        s.sub = s.reduce ? split_candidate(*s.loop) : jitk::get_first_loop_blocks(*s.loop)[1];
+        if (s.reduce)
+            for (const Block &b : s.loop->_block_list) {
+                if (!b.isInstr()) break;
+                folded.insert(b.getInstr().get());
+            }
+        st.push_back(s);
+    }
+    Symbols sym = build_symbols(items, folded);
+    // Instructions over the row (2-D) and after a reduction (1-D), and how every array is touched.
+    struct Use {
+        size_t stage;
+        const bh_view *v;
+        bool write, in_row;
+    };
+    vector<Use> uses;
+    set<const bh_base *> written;
+    for (size_t i = 0; i < st.size(); ++i) {
+        vector<pair<InstrPtr, bool>> instrs;
+        for (const InstrPtr &ip : jitk::all_instr(*st[i].sub)) instrs.emplace_back(ip, true);
+        if (st[i].reduce) {
+            bool after = false;
+            for (const Block &b : st[i].loop->_block_list) {
+                if (!b.isInstr()) after = true;
+                else if (after) instrs.emplace_back(b.getInstr(), false);
+            }
+        }
+        for (const auto &pi : instrs) {
+            const bh_instruction &in = *pi.first;
+            if (bh_opcode_is_system(in.opcode) || in.operand.empty()) continue;
+            if (in.opcode == BH_GATHER || in.opcode == BH_SCATTER || in.opcode == BH_COND_SCATTER ||
+                bh_opcode_is_accumulate(in.opcode))
+                return false;
+            for (size_t o = 1; o < in.operand.size(); ++o)
+                if (!in.operand[o].isConstant()) uses.push_back({i, &in.operand[o], false, pi.second});
+            uses.push_back({i, &in.operand[0], true, pi.second});
+            written.insert(in.operand[0].base);
+        }
+    }
+    struct RowArray {
+        bh_view view;
+        bool load;            // its first use is a read
+        size_t first, last;   // stages that touch it
+        size_t last_write = 0;
+        bool write = false;
+    };
+    map<ViewKey, size_t> row_id;
+    vector<RowArray> rows;
+    map<const bh_base *, pair<int64_t, int64_t>> scalars;  // written per-row values: (start, stride)
+    map<const bh_base *, const bh_view *> row_of;          // written row arrays: their view
+    for (const Use &x : uses) {
+        const bh_base *b = x.v->base;
+        if (sym.temps.count(b)) continue;
+        const bh_view &v = *x.v;
+        const bool two = v.ndim == 2 && x.in_row;
+        if (written.count(b) && x.write) {
+            // a reduction's output and what follows it are one value per row
+            const bool scalar = !two;
+            if (scalar) {
+                if (v.ndim != 1 || v.stride[0] == 0 || row_of.count(b)) return false;
+                const auto at = make_pair(v.start, v.stride[0]);
+                auto it = scalars.emplace(b, at).first;
+                if (it->second != at) return false;
+            } else {
+                if (scalars.count(b) || v.stride[1] == 0 || abs(v.stride[0]) < (len - 1) * abs(v.stride[1]) + 1) return false;
+                row_of.emplace(b, &v);
+            }
+        }
+    }
+    for (const Use &x : uses) {
+        const bh_base *b = x.v->base;
+        if (sym.temps.count(b)) continue;
+        const bh_view &v = *x.v;
+        auto sc = scalars.find(b);
+        if (sc != scalars.end()) {
+            const bool same = v.start == sc->second.first && v.ndim >= 1 && v.stride[0] == sc->second.second &&
+                              (v.ndim == 1 || (v.ndim == 2 && v.stride[1] == 0));
+            if (!same) return false;
+            // a per-row value must be there before it is read: written by an earlier stage or instruction
+            continue;
+        }
+        auto ro = row_of.find(b);
+        if (ro != row_of.end() && !(v == *ro->second)) return false;
+        if (!x.in_row) {
+            if (ro != row_of.end()) return false;
+            continue;  // a 1-D array read after a reduction
+        }
+        if (v.ndim != 2 || v.stride[1] == 0) continue;  // read from memory where it is used
+        auto it = row_id.find(ViewKey(v));
+        if (it == row_id.end()) {
+            it = row_id.emplace(ViewKey(v), rows.size()).first;
+            rows.push_back({v, !x.write, x.stage, x.stage});
+        }
+        rows[it->second].last = x.stage;
+        if (x.write) {
+            rows[it->second].write = true;
+            rows[it->second].last_write = x.stage;
+        }
+    }
+    // Per-row values read before they are written would be another flush's: leave those alone.
+    {
+        set<const bh_base *> seen;
+        for (const Use &x : uses) {
+            if (!scalars.count(x.v->base)) continue;
+            if (x.write) seen.insert(x.v->base);
+            else if (!seen.count(x.v->base)) return false;
+        }
+    }
+    // What one stage alone touches is read and written in memory; the others live in registers from
+    // their first stage to their last. Lanes per row: LANE_REDUCE's, more where a row's part of them
+    // does not fit a lane's registers.
+    rows.erase(remove_if(rows.begin(), rows.end(), [&](const RowArray &r) { return r.first == r.last && !dropped.count(r.view.base); }),
+               rows.end());
+    int live = 0;
+    for (size_t i = 0; i + 1 < st.size(); ++i) {
+        int words = 0;
+        for (const RowArray &r : rows)
+            if (r.first <= i && i < r.last) words += (static_cast<int>(bh_type_size(r.view.base->dtype())) + 3) / 4;
+        live = max(live, words);
+    }
+    if (live == 0) return false;
+    int64_t C = lane_count(points, len);
+    while (C < kThreads && (len + C - 1) / C > kRowElements) C *= 2;
+    const int64_t NU = (len + C - 1) / C;
+    if (C < 2 || NU > kRowElementsMost || NU * live > kRowRegisters) return false;
+    for (const bh_base *b : dropped) sym.temps.insert(b);
+    // Rebuild the parameters without the dropped arrays.
+    {
+        vector<bh_base *> keep;
+        sym.param_id.clear();
+        for (bh_base *b : sym.params)
+            if (!dropped.count(b)) {
+                sym.param_id[b] = static_cast<int>(keep.size());
+                keep.push_back(b);
+            }
+        sym.params = keep;
+    }
+    u = LaunchUnit();
+    u.sched = Sched::ROWS;
+    u.rows = points;
+    u.cols = 1;
+    u.chunks = C;
+    ParamLayout pl;
+    add_common_fields(sym, pl, opt);
+    pl.add(work_field(points), "bh_i64", "points");
+    pl.add(work_field(u.work_items()), "bh_i64", "work");
+    stringstream body;
+    Emitter em(sym, body, opt);
+    const string n1 = "p.n" + to_string(sym.loop_id.at(st[0].sub));
+    // The reductions of every stage, their accumulators and the functions that combine the lanes.
+    struct Red {
+        InstrPtr r;
+        string T, ident, acc;
+    };
+    vector<vector<Red>> reds(st.size());
+    int nred = 0;
+    for (size_t i = 0; i < st.size(); ++i) {
+        vector<InstrPtr> rs(st[i].sub->_sweeps.begin(), st[i].sub->_sweeps.end());
+        sort(rs.begin(), rs.end(), [](const InstrPtr &a, const InstrPtr &b) { return a->origin_id < b->origin_id; });
+        for (const InstrPtr &r : rs) {
+            const bh_type t = r->operand[0].base->dtype();
+            Red x{r, cuda_type(t), constant_literal(jitk::sweep_identity(r->opcode, t)), "racc" + to_string(nred)};
+            u.red_orders.emplace_back(r->origin_id, "lanes:" + to_string(C) + ":" + to_string(len));
+            body << "__device__ __forceinline__ " << x.T << " bh_lanes" << nred << "(" << x.T << " v, unsigned char *sm) {\n";
+            body << "#pragma unroll\n";
+            body << "    for (int m = " << min<int64_t>(C, 32) / 2 << "; m >= 1; m >>= 1) { const " << x.T
+                 << " o = bh_shfl_xor(v, m); v = " << reduce_expr(r->opcode, "v", "o") << "; }\n";
+            if (C <= 32) {
+                // the first lane's value: the trees of the others may order a NaN differently
+                body << "    return bh_shfl_idx(v, (threadIdx.x & 31) & ~" << C - 1 << ");\n";
+            } else {
+                body << "    " << x.T << " *x = (" << x.T << " *)sm;\n";
+                body << "    if ((threadIdx.x & 31) == 0) x[threadIdx.x >> 5] = v;\n";
+                body << "    __syncthreads();\n";
+                body << "    const int w0 = threadIdx.x / " << C << " * " << C / 32 << ";\n";
+                body << "    v = x[w0];\n";
+                body << "#pragma unroll\n";
+                body << "    for (int k = 1; k < " << C / 32 << "; ++k) { const " << x.T << " o = x[w0 + k]; v = "
+                     << reduce_expr(r->opcode, "v", "o") << "; }\n";
+                body << "    __syncthreads();\n";
+                body << "    return v;\n";
+            }
+            body << "}\n";
+            reds[i].push_back(x);
+            ++nred;
+        }
+    }
+    body << "__device__ void bh_work(const P &p, bh_i64 w) {\n";
+    body << pointer_locals(sym);
+    if (C > 32) body << "    __shared__ alignas(16) unsigned char sm[" << kThreads / 32 * 16 << "];\n";
+    else body << "    unsigned char *sm = nullptr;\n";
+    body << "    const int lane = threadIdx.x % " << C << ";\n";
+    body << "    const bh_i64 i0 = w * " << kThreads / C << " + threadIdx.x / " << C << ";\n";
+    body << "    const bool active = i0 < p.points;\n";
+    body << "    const int n = active ? (int)" << n1 << " : 0;\n";
+    // The row pointers of the arrays held in registers.
+    Scope g;
+    for (size_t k = 0; k < rows.size(); ++k) {
+        const bh_view &v = rows[k].view;
+        const string T = cuda_type(v.base->dtype());
+        body << "    " << T << " ra" << k << "[" << NU << "];\n";
+        g.repl[ViewKey(v)] = "ra" + to_string(k) + "[u]";
+        if (dropped.count(v.base)) continue;
+        body << "    " << T << "* __restrict__ rp" << k << " = a" << sym.param_id.at(v.base) << " + "
+             << em.index_expr(v, BH_MAXDIM, {-1, 0}, 1) << ";\n";
+    }
+    auto row_ref = [&](size_t k) { return "rp" + to_string(k) + "[" + em.axis_term(rows[k].view, 1) + "]"; };
+    auto unrolled = [&](const string &inside) {
+        body << "#pragma unroll\n";
+        body << "    for (int u = 0; u < " << NU << "; ++u) {\n";
+        body << "        const int i1 = lane + u * " << C << ";\n";
+        body << "        if (i1 < n) {\n" << inside << "        }\n    }\n";
+    };
+    {
+        string loads;
+        for (size_t k = 0; k < rows.size(); ++k)
+            if (rows[k].load) loads += "            ra" + to_string(k) + "[u] = " + row_ref(k) + ";\n";
+        if (!loads.empty()) unrolled(loads);
+    }
+    // Values per row: reduction results and what instructions after a reduction make of them.
+    map<const bh_base *, string> value;
+    for (const auto &sc : scalars) {
+        const string nm = "rv" + to_string(sym.base_index(sc.first));
+        value[sc.first] = nm;
+        body << "    " << cuda_type(sc.first->dtype()) << " " << nm << ";\n";
+    }
+    for (const Use &x : uses)
+        if (value.count(x.v->base)) g.repl[ViewKey(*x.v)] = value.at(x.v->base);
+    int red_at = 0;
+    for (size_t i = 0; i < st.size(); ++i) {
+        Scope s;
+        s.parent = &g;
+        body << "    {\n";
+        for (Red &r : reds[i]) {
+            body << "    " << r.T << " " << r.acc << " = " << r.ident << ";\n";
+            em.external_acc[ViewKey(r.r->operand[0])] = r.acc;
+        }
+        {
+            stringstream one;
+            Emitter eb(sym, one, opt);
+            eb.external_acc = em.external_acc;
+            Scope in;
+            in.parent = &s;
+            if (!st[i].reduce) {
+                // temporaries of the map's outer rank
+                for (const bh_base *b : eb.sorted_temps(*st[i].loop))
+                    if (sym.temps.count(b) && !dropped.count(b) && !in.is_tmp(b)) {
+                        in.tmps.insert(b);
+                        one << "            " << cuda_type(b->dtype()) << " t" << sym.base_index(b) << ";\n";
+                    }
+            }
+            eb.write_body(*st[i].sub, in, 12);
+            for (size_t k = 0; k < rows.size(); ++k)
+                if (rows[k].write && rows[k].last_write == i && !dropped.count(rows[k].view.base))
+                    one << "            " << row_ref(k) << " = ra" << k << "[u];\n";
+            unrolled(one.str());
+        }
+        for (Red &r : reds[i]) {
+            body << "    " << r.acc << " = bh_lanes" << red_at++ << "(" << r.acc << ", sm);\n";
+            em.external_acc.erase(ViewKey(r.r->operand[0]));
+            const bh_base *b = r.r->operand[0].base;
+            if (value.count(b)) {
+                body << "    " << value.at(b) << " = " << r.acc << ";\n";
+            } else {
+                s.repl[ViewKey(r.r->operand[0])] = r.acc;  // a temporary of this stage
+            }
+        }
+        if (st[i].reduce) {
+            for (const bh_base *b : em.sorted_temps(*st[i].loop)) {
+                bool is_red = false;
+                for (const Red &r : reds[i]) is_red = is_red || r.r->operand[0].base == b;
+                if (sym.temps.count(b) && !dropped.count(b) && !is_red && !s.is_tmp(b)) {
+                    s.tmps.insert(b);
+                    body << "    " << cuda_type(b->dtype()) << " t" << sym.base_index(b) << ";\n";
+                }
+            }
+            bool after = false;
+            stringstream tail;
+            Emitter et(sym, tail, opt);
+            for (const Block &b : st[i].loop->_block_list) {
+                if (!b.isInstr()) after = true;
+                else if (after) et.write_instr(*b.getInstr(), s, 8);
+            }
+            // (1-D arrays other than the row values are only read here)
+            if (!tail.str().empty()) body << "    if (active) {\n" << tail.str() << "    }\n";
+        }
+        body << "    }\n";
+    }
+    string stores;
+    for (const auto &sc : scalars) {
+        if (dropped.count(sc.first)) continue;
+        for (const Use &x : uses)
+            if (x.write && x.v->base == sc.first) {
+                stores += "        " + em.array_ref(*x.v, x.in_row ? 1 : BH_MAXDIM) + " = " + value.at(sc.first) + ";\n";
+                break;
+            }
+    }
+    if (!stores.empty()) body << "    if (active && lane == 0) {\n" << stores << "    }\n";
+    body << "}\n" << kWrappers;
+    u.fields = pl.fields;
+    u.algorithmic_bytes = unit_bytes(sym, items);
+    u.elements = points * len;
+    finish_source(u, pl.decl.str(), body.str(), opt);
+    return true;
+}
+
+// Row fusion over a flush's lowered kernels: the first kernel of each group gets the group's unit,
+// the others' unit lists are emptied and `into` names the first.
+void fuse_rows(const vector<LoopB> &kernels, vector<vector<LaunchUnit>> &lowered, const CodegenOptions &opt, vector<int> &into) {
+    const size_t n = kernels.size();
+    // Kernels that touch each array, and arrays created and freed by the flush.
+    map<const bh_base *, set<size_t>> touches;
+    set<const bh_base *> created, freed;
+    for (size_t k = 0; k < n; ++k) {
+        for (const InstrPtr &ip : jitk::all_instr(kernels[k])) {
+            if (bh_opcode_is_system(ip->opcode)) continue;
+            for (size_t o = 0; o < ip->operand.size(); ++o)
+                if (!ip->operand[o].isConstant()) touches[ip->operand[o].base].insert(k);
+            if (ip->constructor && !ip->operand.empty() && !ip->operand[0].isConstant()) created.insert(ip->operand[0].base);
+        }
+        for (const bh_base *f : kernels[k].getAllFrees()) freed.insert(f);
+    }
+    for (size_t k = 0; k < n; ++k) {
+        RowStage first;
+        if (lowered[k].empty() || !row_stage(kernels[k], lowered[k], first) || first.loop->size < kLaneMinPoints) continue;
+        vector<RowStage> group{first};
+        vector<size_t> members{k};
+        LaunchUnit best;
+        bool have = false;
+        size_t used = 1;
+        bool any_reduce = first.reduce;
+        for (size_t j = k + 1; j < n; ++j) {
+            if (kernels[j].isSystemOnly()) continue;
+            RowStage next;
+            if (!row_stage(kernels[j], lowered[j], next) || next.loop->size != first.loop->size ||
+                next.sub->size != first.sub->size)
+                break;
+            group.push_back(next);
+            members.push_back(j);
+            any_reduce = any_reduce || next.reduce;
+            if (!any_reduce) continue;
+            const set<size_t> in(members.begin(), members.end());
+            set<const bh_base *> dropped;
+            for (const auto &t : touches) {
+                if (!created.count(t.first) || !freed.count(t.first)) continue;
+                bool inside = true;
+                for (size_t m : t.second) inside = inside && in.count(m);
+                if (inside) dropped.insert(t.first);
+            }
+            // something has to be shared: a row array two of the kernels touch
+            bool shared = false;
+            for (const auto &t : touches) {
+                int c = 0;
+                for (size_t m : t.second) c += in.count(m) ? 1 : 0;
+                shared = shared || (c > 1 && t.first->nelem() >= first.loop->size * first.sub->size);
+            }
+            LaunchUnit u;
+            if (shared && lower_rows(group, dropped, opt, u)) {
+                best = std::move(u);
+                have = true;
+                used = group.size();
+            }
+        }
+        if (!have) continue;
+        lowered[k].assign(1, best);
+        for (size_t m = 1; m < used; ++m) {
+            lowered[members[m]].clear();
+            into[members[m]] = static_cast<int>(k);
+        }
+    }
+}
+
 } // namespace
 
 vector<LaunchUnit> lower_kernel(const LoopB &kernel, const CodegenOptions &opt) {
@@ -5215,6 +5656,7 @@ vector<LaunchUnit> lower_kernel(const LoopB &kernel, const CodegenOptions &opt) 
 vector<int> fuse_tails(const vector<LoopB> &kernels, vector<vector<LaunchUnit>> &lowered, const CodegenOptions &opt) {
     vector<int> into(lowered.size(), -1);
     if (opt.bounds_check) return into;
+    if (opt.fuse_rows) fuse_rows(kernels, lowered, opt, into);
     // Bases each kernel reads and writes (frees count as writes).
     const size_t n = kernels.size();
     vector<set<const bh_base *>> reads(n), writes(n);
@@ -5223,6 +5665,14 @@ vector<int> fuse_tails(const vector<LoopB> &kernels, vector<vector<LaunchUnit>> 
             for (size_t o = 0; o < ip->operand.size(); ++o)
                 if (!ip->operand[o].isConstant()) (o == 0 ? writes[k] : reads[k]).insert(ip->operand[o].base);
         for (bh_base *f : kernels[k].getAllFrees()) writes[k].insert(f);
+    }
+    for (size_t k = 0; k < n; ++k) {  // kernels of a row group run at its first one
+        if (into[k] < 0) continue;
+        const size_t h = static_cast<size_t>(into[k]);
+        reads[h].insert(reads[k].begin(), reads[k].end());
+        writes[h].insert(writes[k].begin(), writes[k].end());
+        reads[k].clear();
+        writes[k].clear();
     }
     auto meets = [](const set<const bh_base *> &a, const set<const bh_base *> &b) {
         for (const bh_base *x : a)

@@ -35,6 +35,9 @@
 //   AXIS_SCAN     an accumulate along an axis of an array of two or more dimensions: a thread per
 //                 point (or a warp, when the axis is contiguous), the axis cut into chunks in two
 //                 units (chunk totals, scan) when the points alone are few.
+//   ROWS          several neighbouring kernels over the rows of one index space (row reductions and
+//                 maps) whose arrays meet in the same row only: C lanes hold a row in registers (see
+//                 fuse_rows).
 //   SERIAL        anything else: one thread runs the nest in program order (always correct).
 //   TILE2D        a 2-D map that reads arrays through transposed views (unit stride along the outer
 //                 rank): tiles of (128 bytes / element) rows x 64 columns; each transposed view's
@@ -60,7 +63,7 @@
 namespace bohrium {
 namespace cuda {
 
-enum class Sched { FLAT, GRID_REDUCE, SPLIT_REDUCE, LANE_REDUCE, OUTER_REDUCE, SCAN1D, SERIAL, TILE2D, AXIS_SCAN };
+enum class Sched { FLAT, GRID_REDUCE, SPLIT_REDUCE, LANE_REDUCE, OUTER_REDUCE, SCAN1D, SERIAL, TILE2D, AXIS_SCAN, ROWS };
 
 // Engine-internal opcodes made by contract_multiply_add() (contract.cpp), operands (out, a, b, c):
 //   BH_X_FMA   out = a*b + c      BH_X_FMS   out = a*b - c      BH_X_FNMA  out = c - a*b
@@ -127,7 +130,7 @@ struct LaunchUnit {
     int nred = 0;               // GRID_REDUCE / SPLIT_REDUCE: number of reductions
     int64_t scratch_bytes_per_tile = 0; // GRID_REDUCE: bytes of partials per tile (all reductions)
     int slot_bytes = 8;         // GRID_REDUCE / SPLIT_REDUCE: bytes of one partial (16 with complex128)
-    int64_t chunks = 1;         // SPLIT_REDUCE: chunks of the swept axis; LANE_REDUCE: lanes per point;
+    int64_t chunks = 1;         // SPLIT_REDUCE: chunks of the swept axis; LANE_REDUCE, ROWS: lanes per point;
                                 // GRID_REDUCE: tiles per work item; SCAN1D, AXIS_SCAN: work items of the phase
     int64_t batch_chunks = 0;   // GRID_REDUCE: tiles per work item in a grouped launch (0: chunks)
     int64_t scan_bytes = 0;     // SCAN1D: its chunk totals and carries and group totals and carries;
@@ -171,6 +174,7 @@ struct CodegenOptions {
     bool scan_single_pass = false; // SCAN1D as one pass with look-back (else three units; see lower_scan1d_single)
     bool scan_windows = false;     // SCAN1D units A and C one group of chunks at a time (see lower_scan1d)
     bool stage_bulk = true;        // LANE_REDUCE stencil rows staged by TMA bulk copies (else cp.async)
+    bool fuse_rows = true;         // neighbouring row-wise kernels of a flush run as one (ROWS)
     bool scan_prefetch = true;     // SCAN1D streaming units read their inputs from a TMA-filled ring
     int64_t scan_spin_cap = int64_t{1} << 22; // polls per look-back wait (negative: give up at once)
 };

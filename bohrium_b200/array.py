@@ -8,6 +8,7 @@ bridge does on GPU stacks (bridge/npbackend/bohrium/ufuncs.pyx:371-440).
 """
 from __future__ import annotations
 
+import math
 import numbers
 from typing import Optional, Sequence
 
@@ -34,8 +35,8 @@ class BhArray:
         self.rt = rt
         self.base = base
         self.start = int(start)
-        self.shape = tuple(int(s) for s in shape)
-        self.strides = tuple(int(s) for s in strides)
+        self.shape = tuple(map(int, shape))
+        self.strides = tuple(map(int, strides))
         self._owner = owner  # the array owning `base` (None: this array owns it)
 
     def __del__(self):
@@ -56,7 +57,7 @@ class BhArray:
 
     @property
     def size(self):
-        return int(np.prod(self.shape, dtype=np.int64)) if self.shape else 1
+        return math.prod(self.shape)
 
     def view(self) -> ir.View:
         # Zero-dimensional arrays travel as one-element 1-D views, as the reference's bridge sends
@@ -240,8 +241,7 @@ class BhArray:
 # ------------------------------------------------------------------------------ construction
 def empty(rt: Runtime, shape, dtype=np.float64) -> BhArray:
     shape = (shape,) if isinstance(shape, numbers.Integral) else tuple(shape)
-    n = int(np.prod(shape, dtype=np.int64)) if shape else 1
-    base = rt.new_base(dtype, n)
+    base = rt.new_base(dtype, int(math.prod(shape)))
     return BhArray(rt, base, 0, shape, _contig_strides(shape))
 
 
@@ -293,7 +293,7 @@ def _result_type(a, b):
     ta = a.dtype if isinstance(a, BhArray) else None
     tb = b.dtype if isinstance(b, BhArray) else None
     if ta is not None and tb is not None:
-        return np.result_type(ta, tb)
+        return ta if ta is tb else np.result_type(ta, tb)
     t = ta if ta is not None else tb
     s = b if ta is not None else a
     if isinstance(s, (bool, np.bool_)):
@@ -309,18 +309,25 @@ def _result_type(a, b):
     return np.result_type(t, np.asarray(s).dtype)
 
 
+_FLOAT64 = np.dtype(np.float64)
+
+
 def _operand(x, dtype, shape):
     if isinstance(x, BhArray):
-        if x.dtype != dtype:
+        if x.dtype is not dtype and x.dtype != dtype:
             x = x.astype(dtype)
         return x._broadcast_to(shape), None
+    if type(x) is float and dtype == _FLOAT64:
+        return None, ir.Constant(x, ir.FLOAT64)
     return None, ir.Constant(np.asarray(x).astype(dtype).item() if dtype != np.bool_ else bool(x), ir.bh_type(dtype))
 
 
 def binary(name: str, a, b, out_dtype=None, out: Optional[BhArray] = None) -> BhArray:
     rt = a.rt if isinstance(a, BhArray) else b.rt
     dtype = _result_type(a, b)
-    shape = np.broadcast_shapes(a.shape if isinstance(a, BhArray) else (), b.shape if isinstance(b, BhArray) else ())
+    sa = a.shape if isinstance(a, BhArray) else ()
+    sb = b.shape if isinstance(b, BhArray) else ()
+    shape = sa if sa == sb or not sb else sb if not sa else np.broadcast_shapes(sa, sb)
     if out is None:
         out = empty(rt, shape, out_dtype if out_dtype is not None else dtype)
     va, ca = _operand(a, dtype, shape)

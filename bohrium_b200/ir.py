@@ -7,9 +7,11 @@ bhb_ir_create() in include/bh_b200.h.
 """
 from __future__ import annotations
 
+import array
 import itertools
+import struct
 from dataclasses import dataclass, field
-from typing import Optional, Sequence
+from typing import NamedTuple, Optional, Sequence
 
 import numpy as np
 
@@ -77,8 +79,7 @@ class Base:
         return f"a{self.id}<{self.dtype},{self.nelem}>"
 
 
-@dataclass(frozen=True)
-class View:
+class View(NamedTuple):
     base: Base
     start: int
     shape: tuple
@@ -99,6 +100,10 @@ class Constant:
     dtype: int  # bh_type
 
     def words(self) -> tuple:
+        if self.dtype == FLOAT64 and type(self.value) is float:
+            return _ONE_WORD.unpack(_FLOAT64.pack(self.value))[0], 0
+        if self.dtype == INT64 and type(self.value) is int and -(1 << 63) <= self.value < 1 << 63:
+            return self.value, 0
         raw = bytearray(16)
         if self.dtype == R123:
             start, key = self.value
@@ -108,8 +113,10 @@ class Constant:
             arr = np.array([self.value], dtype=np_dtype(self.dtype))
             b = arr.tobytes()
             raw[: len(b)] = b
-        w = np.frombuffer(bytes(raw), dtype=np.int64)
-        return int(w[0]), int(w[1])
+        return _TWO_WORDS.unpack(raw)
+
+
+_FLOAT64, _ONE_WORD, _TWO_WORDS = struct.Struct("<d"), struct.Struct("<q"), struct.Struct("<qq")
 
 
 @dataclass
@@ -150,21 +157,23 @@ def encode(instrs: Sequence[Instr]) -> np.ndarray:
     """Encode instructions into the int64 words read by bhb_ir_create()."""
     words: list = []
     for ins in instrs:
-        if ins.constant is not None:
-            c0, c1 = ins.constant.words()
-            words += [ins.opcode, len(ins.operands), ins.constant.dtype, c0, c1]
+        operands, constant = ins.operands, ins.constant
+        if constant is not None:
+            c0, c1 = constant.words()
+            words += (ins.opcode, len(operands), constant.dtype, c0, c1)
         else:
-            words += [ins.opcode, len(ins.operands), -1, 0, 0]
-        for op in ins.operands:
+            words += (ins.opcode, len(operands), -1, 0, 0)
+        for op in operands:
             if op is None:
                 words.append(0)
             else:
-                if op.base.handle == 0:
-                    raise RuntimeError(f"base {op.base} has no native handle")
-                words += [op.base.handle, op.start, len(op.shape)]
-                words += list(op.shape)
-                words += list(op.stride)
-    return np.array(words, dtype=np.int64)
+                base, start, shape, stride = op
+                if base.handle == 0:
+                    raise RuntimeError(f"base {base} has no native handle")
+                words += (base.handle, start, len(shape))
+                words += shape
+                words += stride
+    return np.frombuffer(array.array("q", words), dtype=np.int64)
 
 
 def encode_slides(instrs: Sequence[Instr]) -> np.ndarray:

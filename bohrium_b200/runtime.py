@@ -10,7 +10,6 @@ from __future__ import annotations
 
 import ctypes
 import os
-import weakref
 from typing import Optional
 
 import numpy as np
@@ -219,7 +218,6 @@ class Runtime:
     def new_base(self, dtype, nelem: int) -> ir.Base:
         b = ir.Base(dtype, nelem)
         self.ex.register(b)
-        weakref.finalize(b, lambda: None)
         return b
 
     def enqueue(self, ins: ir.Instr) -> None:

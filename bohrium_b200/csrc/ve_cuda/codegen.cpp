@@ -3157,6 +3157,9 @@ string block_reduce_k_fn(const string &ctype, const string &fname, bh_opcode op,
     return ss.str();
 }
 
+// Tiles from which heavy bodies take half tiles (emit_half_tiles): fewer run at once on the GPU
+// whatever their registers, and then a second wait for memory costs more.
+constexpr int64_t kHalfTiles = 148 * 3;
 LaunchUnit lower_grid_reduce(const LoopB &loop, const vector<InstrPtr> &identities, const CodegenOptions &opt,
                              int forceK = 0) {
     LaunchUnit u;
@@ -3436,7 +3439,7 @@ LaunchUnit lower_grid_reduce(const LoopB &loop, const vector<InstrPtr> &identiti
         Emitter eb(sym, body, opt);
         eb.external_acc = acc_k;
         if (vectorized) emit_vec_check(eb);
-        if (heavy && vectorized && K == 1) {
+        if (heavy && vectorized && K == 1 && ntiles > kHalfTiles) {
             emit_half_tiles(eb);
         } else {
         if (!pre.empty()) {
@@ -5089,11 +5092,10 @@ struct P {
     bh_u2::P b;
     alignas(8) unsigned int* tail_counter;
 };
-// Every thread's writes are made visible device-wide, thread 0 arrives with an acquire-release
-// atomic, and the tail's threads acquire before reading.
+// The barrier orders every thread's writes before thread 0's acquire-release arrival, which makes
+// them visible device-wide (release is cumulative); the tail's threads acquire before reading.
 __device__ __forceinline__ bool bh_tail_gate(unsigned int *counter, unsigned int arrivals) {
     __shared__ bool last;
-    __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) last = bh_arrive(counter) == arrivals - 1u;
     __syncthreads();

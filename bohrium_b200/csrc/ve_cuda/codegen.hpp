@@ -7,7 +7,8 @@
 //
 //   FLAT          the leading parallel ranks form a (rows x cols) index space processed by a
 //                 grid-stride persistent kernel, V elements per thread along the innermost
-//                 parallel rank; deeper ranks are serial loops inside the thread.
+//                 parallel rank (or, for short rows, along the two innermost walked as one); deeper
+//                 ranks are serial loops inside the thread.
 //   GRID_REDUCE   a 1-D nest that reduces its only axis (maps fused with sum/max/... to a scalar):
 //                 fixed tiles of TILE = 256 x 8 elements, a per-tile CTA tree, then the last CTA
 //                 folds the tile partials in tile order. The summation order depends only on the
@@ -124,7 +125,7 @@ struct LaunchUnit {
     std::string name;   // kernel function name (derived from the source hash)
     std::string source; // complete CUDA source
     Sched sched = Sched::FLAT;
-    int V = 1;          // elements per thread along the innermost parallel rank (FLAT)
+    int V = 1;          // elements per thread along the innermost parallel rank (FLAT); SPLIT_REDUCE: points per CTA
     std::vector<ParamField> fields;
     int64_t rows = 1, cols = 1; // FLAT / OUTER_REDUCE index space; GRID_REDUCE/SCAN1D: cols = length
     int nred = 0;               // GRID_REDUCE / SPLIT_REDUCE: number of reductions

@@ -1982,7 +1982,8 @@ bool lower_tile2d(const LoopB &loop, const CodegenOptions &opt, LaunchUnit &u) {
         pl.pad64();
     }
 
-    const string T = cuda_type(tv[0].base->dtype());
+    vector<string> T;  // the views share an element size, not a type
+    for (const bh_view &v : tv) T.push_back(cuda_type(v.base->dtype()));
     const string rows = "p.n" + to_string(sym.loop_id.at(&L)), cols = "p.n" + to_string(sym.loop_id.at(&inner));
     stringstream body;
     if (tma) body << "// bh_dynamic_shared_bytes: " << stages * static_cast<int>(tv.size()) * kTileBoxBytes + 1024 << "\n";
@@ -1994,10 +1995,10 @@ bool lower_tile2d(const LoopB &loop, const CodegenOptions &opt, LaunchUnit &u) {
     body << "    const bh_i64 i1 = tc * 64 + c;\n";
     body << "    const bh_i64 rbase = tr * " << TR << " + rq * " << RPT << ";\n";
     for (size_t k = 0; k < tv.size(); ++k) {
-        body << "    " << T << " tv" << k << "[" << RPT << "];\n";
+        body << "    " << T[k] << " tv" << k << "[" << RPT << "];\n";
         if (!tpose[k]) {
             // row-wise: row r of the tile at r * 64 elements, read in the element loop
-            body << "    const " << T << " *tr" << k << " = (const " << T << " *)(stage + " << k * kTileBoxBytes
+            body << "    const " << T[k] << " *tr" << k << " = (const " << T[k] << " *)(stage + " << k * kTileBoxBytes
                  << ") + (rq * " << RPT << ") * 64 + c;\n";
             continue;
         }
@@ -2015,8 +2016,8 @@ bool lower_tile2d(const LoopB &loop, const CodegenOptions &opt, LaunchUnit &u) {
         Emitter es(sym, body, opt);
         body << "    if (!STAGED) {\n";
         for (size_t k = 0; k < tv.size(); ++k) {
-            body << "        " << T << " ld" << k << "[" << RPT << "];\n";
-            if (tpose[k]) body << "        __shared__ " << T << " box" << k << "[" << kTileCols * (TR + 1) << "];\n";
+            body << "        " << T[k] << " ld" << k << "[" << RPT << "];\n";
+            if (tpose[k]) body << "        __shared__ " << T[k] << " box" << k << "[" << kTileCols * (TR + 1) << "];\n";
         }
         body << "#pragma unroll\n";
         body << "        for (int e = 0; e < " << RPT << "; ++e) {\n";

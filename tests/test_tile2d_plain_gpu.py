@@ -27,3 +27,30 @@ def test_transposed_operands(gpu_executor, shape, dtype, mode):
         gpu_executor.message("CUDA: batch off")
     for g, w in zip(got, [A + B.T, A - C.T, B.T + C.T, A[1:, 1:] + B[1:, 1:].T]):
         np.testing.assert_array_equal(g, w)
+
+
+@pytest.mark.parametrize("types", [(np.float32, np.int32), (np.int32, np.float32), (np.uint32, np.float32),
+                                   (np.float64, np.int64), (np.int64, np.float64)])
+@pytest.mark.parametrize("shape", [(65, 99), (256, 320), (517, 301)])
+@pytest.mark.parametrize("mode", ["off", "grouped"])
+def test_operands_of_two_types(gpu_executor, types, shape, mode):
+    """One element size, two types, on every way into the tile (256 x 320: tensor maps)."""
+    ta, tb = types
+    to = ta if np.issubdtype(ta, np.floating) else tb
+    rng = np.random.default_rng(1)
+    A = rng.integers(0, 99, shape).astype(ta)
+    B = rng.integers(0, 99, shape[::-1]).astype(tb)
+    if np.issubdtype(ta, np.floating):
+        A += ta(0.5)
+    if np.issubdtype(tb, np.floating):
+        B += tb(0.5)
+    gpu_executor.message("CUDA: batch " + mode)
+    try:
+        rt = bh.Runtime(gpu_executor)
+        a, b = bh.array(rt, A), bh.array(rt, B)
+        rt.flush()
+        out = a.astype(to) + b.T.astype(to)
+        got = out.numpy()
+    finally:
+        gpu_executor.message("CUDA: batch off")
+    np.testing.assert_array_equal(got, A.astype(to) + B.T.astype(to))

@@ -2012,24 +2012,42 @@ bool lower_tile2d(const LoopB &loop, const CodegenOptions &opt, LaunchUnit &u) {
     }
     // Without TMA the boxes go through shared memory all the same: neighbouring threads load
     // neighbouring elements of a base row (TR of them), all loads of the tile before the barrier.
+    // Full tiles load without bounds checks, from pointers that step along the tile: with a 64-bit
+    // index and two comparisons per load the address arithmetic bound the kernel (8191 x 6001
+    // float32 on a B200: 133 to 140 us, now 103; 1001 x 999 10.8 and 9.0 us). Issuing the next
+    // tile's loads before this one is computed gained nothing (134 us), 64 rows a tile less (140).
     {
         Emitter es(sym, body, opt);
+        const string full = "tr * " + to_string(TR) + " + " + to_string(TR) + " <= " + rows + " && tc * " + to_string(kTileCols) +
+                            " + " + to_string(kTileCols) + " <= " + cols;
         body << "    if (!STAGED) {\n";
         for (size_t k = 0; k < tv.size(); ++k) {
-            body << "        " << T[k] << " ld" << k << "[" << RPT << "];\n";
-            if (tpose[k]) body << "        __shared__ " << T[k] << " box" << k << "[" << kTileCols * (TR + 1) << "];\n";
-        }
-        body << "#pragma unroll\n";
-        body << "        for (int e = 0; e < " << RPT << "; ++e) {\n";
-        for (size_t k = 0; k < tv.size(); ++k) {
-            body << "            {\n";
+            const string K = to_string(k);
+            body << "        " << T[k] << " ld" << K << "[" << RPT << "];\n";
+            if (tpose[k]) body << "        __shared__ " << T[k] << " box" << K << "[" << kTileCols * (TR + 1) << "];\n";
+            body << "        const " << T[k] << " *q" << K << ";\n        bh_i64 qs" << K << ";\n";
             if (tpose[k]) {
-                body << "                const int at = e * " << kThreads << " + threadIdx.x;\n";
-                body << "                const bh_i64 i0 = tr * " << TR << " + at % " << TR << ", i1 = tc * 64 + at / " << TR << ";\n";
+                body << "        { const bh_i64 i0 = tr * " << TR << " + threadIdx.x % " << TR << ", i1 = tc * " << kTileCols
+                     << " + threadIdx.x / " << TR << "; q" << K << " = &" << es.array_ref(tv[k]) << "; }\n";
+                body << "        { const bh_i64 i1 = " << kThreads / TR << "; qs" << K << " = " << es.axis_term(tv[k], 1) << "; }\n";
             } else {
-                body << "                const bh_i64 i0 = rbase + e;\n";
+                body << "        { const bh_i64 i0 = rbase; q" << K << " = &" << es.array_ref(tv[k]) << "; }\n";
+                body << "        { const bh_i64 i0 = 1; qs" << K << " = " << es.axis_term(tv[k], 0) << "; }\n";
             }
-            body << "                if (i0 < " << rows << " && i1 < " << cols << ") ld" << k << "[e] = " << es.array_ref(tv[k]) << ";\n";
+        }
+        for (int path = 0; path < 2; ++path) {
+            body << (path == 0 ? "        if (" + full + ") {\n" : string("        } else {\n"));
+            body << "#pragma unroll\n";
+            body << "            for (int e = 0; e < " << RPT << "; ++e) {\n";
+            for (size_t k = 0; k < tv.size(); ++k) {
+                body << "                ";
+                if (path == 1 && tpose[k])
+                    body << "if (tr * " << TR << " + threadIdx.x % " << TR << " < " << rows << " && tc * " << kTileCols << " + e * "
+                         << kThreads / TR << " + threadIdx.x / " << TR << " < " << cols << ") ";
+                else if (path == 1)
+                    body << "if (rbase + e < " << rows << " && i1 < " << cols << ") ";
+                body << "ld" << k << "[e] = *q" << k << ";\n                q" << k << " += qs" << k << ";\n";
+            }
             body << "            }\n";
         }
         body << "        }\n";

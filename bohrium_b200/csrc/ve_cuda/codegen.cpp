@@ -1867,11 +1867,14 @@ LaunchUnit lower_flat(const LoopB &loop, unsigned P, const CodegenOptions &opt) 
 // rows. Here a work item is a tile of TR rows x 64 columns of the index space, TR = 128 bytes /
 // element size; thread t handles column t % 64 and rows (t / 64) * TR/4 ... + TR/4 - 1, so each
 // output row of the tile is written by consecutive threads. A transposed view's part of a tile is
-// a TR x 64 box of its base array (64 rows of 128 contiguous bytes), brought into a 4-stage
-// shared-memory ring by one TMA copy per tile, up to 4 tiles ahead, with the 128-byte swizzle; a
+// a TR x 64 box of its base array (64 rows of 128 contiguous bytes), brought into a 2-stage
+// shared-memory ring by one TMA copy per tile, up to 2 tiles ahead, with the 128-byte swizzle; a
 // thread reads its TR/4 values as two 16-byte words (distinct banks across every 8 threads).
 constexpr int kTileCols = 64;
-constexpr int kTileStages = 4;
+// Two stages: 32 KB for two views, so six CTAs fit on an SM. Four stages and three CTAs hold the
+// same bytes in flight with half the warps to store them (float32 8192 x 6000 on a B200: 115 and
+// 108 us, 2048 x 2048 13.9 and 11.9 us, 8192 x 8192 148 and 144 us).
+constexpr int kTileStages = 2;
 constexpr int kTileBoxBytes = kTileCols * 128;
 
 // The views of `inner` that TILE2D stages: first the transposed ones -- read-only (their base is
@@ -1933,7 +1936,7 @@ bool lower_tile2d(const LoopB &loop, const CodegenOptions &opt, LaunchUnit &u) {
     vector<bool> tpose;
     const vector<bh_view> tv = tile2d_views(L, inner, sym, opt, tpose);
     if (tv.empty()) return false;
-    const int stages = tv.size() <= 2 ? kTileStages : kTileStages - 1;
+    const int stages = kTileStages;
     const int esize = bh_type_size(tv[0].base->dtype());
     const int TR = 128 / esize, RPT = TR / 4;  // rows per tile, rows per thread
     u = LaunchUnit();
@@ -1943,7 +1946,7 @@ bool lower_tile2d(const LoopB &loop, const CodegenOptions &opt, LaunchUnit &u) {
     u.cols = inner.size;
     const int64_t tiles_c = (u.cols + kTileCols - 1) / kTileCols;
     // Rows or starts off the 16-byte boundary rule TMA out for every array of this shape: the unit
-    // then has no tensor maps and no ring, whose 64 KB would leave three CTAs on an SM.
+    // then has no tensor maps and no ring.
     bool tma = true;
     for (size_t k = 0; k < tv.size(); ++k) {
         const int64_t ld = tpose[k] ? tv[k].stride[1] : tv[k].stride[0];

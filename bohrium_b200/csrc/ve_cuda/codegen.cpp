@@ -3278,10 +3278,10 @@ LaunchUnit lower_grid_reduce(const LoopB &loop, const vector<InstrPtr> &identiti
     // slot k, elements j = 0..7 in order, in both paths.
     const string n0 = "p.n" + to_string(sym.loop_id.at(&L));
     const bool heavy = heavy_body(L);
-    // Loading every element's inputs up front keeps K x 8 loads in flight. A heavy body pays for
-    // them in registers (Black-Scholes: 80 and 3 CTAs per SM with them, 48 and 5 without) and is
-    // still faster with them (0.174 vs 0.188 ms per 10M options on a B200), so `preload_heavy`
-    // is on by default.
+    // Loading every element's inputs up front keeps K x 8 loads in flight, at the cost of registers
+    // in a heavy body. Black-Scholes on whole tiles was faster with them (0.174 and 0.188 ms per 10M
+    // options on a B200) and is as fast either way on half tiles (163 and 162 us): `preload_heavy`
+    // is on by default for the sizes that run whole tiles.
     const vector<bh_view> pre = heavy && !opt.preload_heavy ? vector<bh_view>{} : preloadable_views(L, L, sym);
     map<ViewKey, string> acc_k;
     for (size_t k = 0; k < reds.size(); ++k) acc_k[ViewKey(reds[k]->operand[0])] = accs[k] + "[k]";

@@ -3603,20 +3603,24 @@ LaunchUnit lower_grid_reduce(const LoopB &loop, const vector<InstrPtr> &identiti
     // or for an atomic's round trip (one of each per tile before: pi from 5e7 random points 231 us, now
     // 203; the plain chain of 2^20 float64 17.2 and 15.4 us).
     int64_t warp_bytes = 0;
-    vector<int64_t> warp_off;
-    for (size_t k = 0; k < reds.size(); ++k) {
-        warp_off.push_back(warp_bytes);
-        warp_bytes += (kThreads / 32) * bh_type_size(reds[k]->operand[0].base->dtype());
-    }
+    for (const InstrPtr &r : reds) warp_bytes += (kThreads / 32) * bh_type_size(r->operand[0].base->dtype());
     const int64_t held = max<int64_t>(K, min<int64_t>(64, 8192 / warp_bytes) / K * K);
+    // Each reduction's slots start on a 16-byte boundary: the largest element alignment, whatever
+    // the types before it and the number of tiles held.
+    vector<int64_t> warp_off;
+    int64_t held_bytes = 0;
+    for (const InstrPtr &r : reds) {
+        warp_off.push_back(held_bytes);
+        held_bytes += (held * (kThreads / 32) * bh_type_size(r->operand[0].base->dtype()) + 15) / 16 * 16;
+    }
     body << "__device__ __forceinline__ void bh_main(const P &p) {\n";
     body << pointer_locals(sym);
     body << "    __shared__ alignas(16) unsigned long long sm_raw[" << (sm_bytes + 7) / 8 << "];\n";
-    body << "    __shared__ alignas(16) unsigned char warp_sm[" << (held * warp_bytes + 15) / 16 * 16 << "];\n";
+    body << "    __shared__ alignas(16) unsigned char warp_sm[" << held_bytes << "];\n";
     body << "    __shared__ bool am_last;\n";
     emit_partials();
     for (size_t k = 0; k < reds.size(); ++k)
-        body << "    " << ctypes[k] << "* ws" << k << " = (" << ctypes[k] << "*)(warp_sm + " << held * warp_off[k] << ");\n";
+        body << "    " << ctypes[k] << "* ws" << k << " = (" << ctypes[k] << "*)(warp_sm + " << warp_off[k] << ");\n";
     body << "    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;\n";
     body << "    int held = 0;\n";
     body << "    for (bh_i64 w = blockIdx.x; w < p.work; w += gridDim.x) {\n";

@@ -3615,8 +3615,11 @@ LaunchUnit lower_grid_reduce(const LoopB &loop, const vector<InstrPtr> &identiti
     }
     body << "__device__ __forceinline__ void bh_main(const P &p) {\n";
     body << pointer_locals(sym);
-    body << "    __shared__ alignas(16) unsigned long long sm_raw[" << (sm_bytes + 7) / 8 << "];\n";
-    body << "    __shared__ alignas(16) unsigned char warp_sm[" << held_bytes << "];\n";
+    // The last CTA's block trees use the same memory: its warp trees have been read by then. (Two
+    // arrays passed the 48 KB of static shared memory at 200 complex128 or 400 float64 reductions,
+    // which one kernel holds otherwise.)
+    body << "    __shared__ alignas(16) unsigned char warp_sm[" << max<int64_t>(held_bytes, (kThreads / 32) * u.slot_bytes) << "];\n";
+    body << "    unsigned char *sm_raw = warp_sm;\n";
     body << "    __shared__ bool am_last;\n";
     emit_partials();
     for (size_t k = 0; k < reds.size(); ++k)

@@ -47,6 +47,21 @@ def test_every_reduction_has_aligned_slots_of_its_own(count):
         assert end <= size, (dtypes, regions, size)
 
 
+@pytest.mark.parametrize("dtype,count", [(np.float64, 400), (np.complex128, 200), (np.float64, 3)])
+def test_shared_memory_of_many_reductions(dtype, count):
+    """A plain launch's shared memory grows by one set of slots a reduction: what it needs beside the
+    warps' slots lies in the same array, so a kernel of many reductions stays below 48 KB."""
+    rt = bh.Runtime(bh.DryRunExecutor())
+    arrays = [bh.empty(rt, (5000,), dtype) for _ in range(count)]
+    keep = [a.sum() for a in arrays]
+    (unit,) = [u for k in bh.dry_run(rt.take(), compile=False)["kernels"] for u in k["units"]]
+    assert len(keep) == count
+    main = unit["source"].split("void bh_main(const P &p)")[1].split("\n}\n")[0]
+    declared = [(t, int(n)) for t, n in re.findall(r"__shared__ (?:alignas\(\d+\) )?([\w ]+?) \w+\[(\d+)\]", main)]
+    size = {"unsigned char": 1, "unsigned long long": 8}
+    assert sum(size[t] * n for t, n in declared) <= 48 * 1024 - 64
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("wide", [2, 4])
 @pytest.mark.parametrize("narrow", [np.int8, np.bool_])

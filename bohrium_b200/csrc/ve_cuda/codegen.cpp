@@ -5258,8 +5258,8 @@ bool row_stage(const LoopB &kernel, const vector<LaunchUnit> &units, RowStage &s
 }
 
 // Lowers `stages` (the kernels' loops, in order) as one unit; false when they are not row-local or
-// too large. `dropped`: arrays that nothing outside the group sees.
-bool lower_rows(const vector<RowStage> &stages, const set<const bh_base *> &dropped, const CodegenOptions &opt, LaunchUnit &u) {
+// too large. `unseen`: arrays that nothing outside the group sees.
+bool lower_rows(const vector<RowStage> &stages, const set<const bh_base *> &unseen, const CodegenOptions &opt, LaunchUnit &u) {
     const int64_t points = stages[0].loop->size, len = stages[0].sub->size;
     vector<Block> holders;
     holders.reserve(stages.size());
@@ -5281,6 +5281,11 @@ bool lower_rows(const vector<RowStage> &stages, const set<const bh_base *> &drop
         st.push_back(s);
     }
     Symbols sym = build_symbols(items, folded);
+    // The arrays that the group keeps from memory. A kernel's own temporaries are not among them:
+    // they stay registers of their stage.
+    set<const bh_base *> dropped;
+    for (const bh_base *b : unseen)
+        if (!sym.temps.count(b)) dropped.insert(b);
     // Instructions over the row (2-D) and after a reduction (1-D), and how every array is touched.
     struct Use {
         size_t stage;
@@ -5614,12 +5619,12 @@ void fuse_rows(const vector<LoopB> &kernels, vector<vector<LaunchUnit>> &lowered
             any_reduce = any_reduce || next.reduce;
             if (!any_reduce) continue;
             const set<size_t> in(members.begin(), members.end());
-            set<const bh_base *> dropped;
+            set<const bh_base *> unseen;
             for (const auto &t : touches) {
                 if (!created.count(t.first) || !freed.count(t.first)) continue;
                 bool inside = true;
                 for (size_t m : t.second) inside = inside && in.count(m);
-                if (inside) dropped.insert(t.first);
+                if (inside) unseen.insert(t.first);
             }
             // something has to be shared: a row array two of the kernels touch
             bool shared = false;
@@ -5629,7 +5634,7 @@ void fuse_rows(const vector<LoopB> &kernels, vector<vector<LaunchUnit>> &lowered
                 shared = shared || (c > 1 && t.first->nelem() >= first.loop->size * first.sub->size);
             }
             LaunchUnit u;
-            if (shared && lower_rows(group, dropped, opt, u)) {
+            if (shared && lower_rows(group, unseen, opt, u)) {
                 best = std::move(u);
                 have = true;
                 used = group.size();

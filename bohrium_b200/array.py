@@ -240,8 +240,9 @@ class BhArray:
 
 # ------------------------------------------------------------------------------ construction
 def empty(rt: Runtime, shape, dtype=np.float64) -> BhArray:
-    shape = (shape,) if isinstance(shape, numbers.Integral) else tuple(shape)
-    base = rt.new_base(dtype, int(math.prod(shape)))
+    # Python integers: a product of NumPy's would wrap in their type
+    shape = (int(shape),) if isinstance(shape, numbers.Integral) else tuple(map(int, shape))
+    base = rt.new_base(dtype, math.prod(shape))
     return BhArray(rt, base, 0, shape, _contig_strides(shape))
 
 

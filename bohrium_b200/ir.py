@@ -173,7 +173,10 @@ def encode(instrs: Sequence[Instr]) -> np.ndarray:
                 words += (base.handle, start, len(shape))
                 words += shape
                 words += stride
-    return np.frombuffer(array.array("q", words), dtype=np.int64)
+    try:
+        return np.frombuffer(array.array("q", words), dtype=np.int64)
+    except TypeError:  # starts, shapes or strides that are whole floats
+        return np.array(words, dtype=np.int64)
 
 
 def encode_slides(instrs: Sequence[Instr]) -> np.ndarray:

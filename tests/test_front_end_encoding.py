@@ -46,3 +46,20 @@ def test_broadcast_shapes_and_result_types(sa, sb):
     for t, k, want in [(np.int32, 2.5, np.float64), (np.float32, 2.5, np.float32), (np.int64, True, np.int64), (np.float32, 1j, np.complex64)]:
         assert bh.binary("ADD", bh.empty(rt, (4,), t), k).dtype == want
     assert bh.empty(rt, (0, 5)).size == 0 and bh.empty(rt, ()).size == 1
+
+
+@pytest.mark.parametrize("t", [np.int8, np.int16, np.int32, np.uint8, np.int64])
+def test_shapes_of_narrow_integers(t):
+    """Element counts and strides of shapes given in NumPy integers do not wrap in their type."""
+    rt = bh.Runtime(bh.DryRunExecutor())
+    side = {1: 100, 2: 30_000, 4: 70_000, 8: 70_000}[np.dtype(t).itemsize]
+    a = bh.empty(rt, (t(side), t(side), t(3)), np.int8)
+    assert a.base.nelem == side * side * 3 and a.strides == (side * 3, 3, 1) and a.size == a.base.nelem
+    assert bh.empty(rt, t(5)).shape == (5,) and bh.empty(rt, np.array([3, 4], dtype=t)).base.nelem == 12
+
+
+def test_views_given_in_whole_floats_still_encode():
+    base = ir.Base(np.float64, 12)
+    base.handle = 77
+    ins = ir.Instr(ir.OPCODES["IDENTITY"], [ir.View(base, 2.0, (4.0,), (1,)), None], ir.Constant(1.0, ir.FLOAT64))
+    assert ir.encode([ins]).tolist()[-6:] == [77, 2, 1, 4, 1, 0]

@@ -906,9 +906,10 @@ public:
     }
 
     string name(const bh_view &v, const Scope &s, int hidden_axis = BH_MAXDIM) {
-        if (s.is_tmp(v.base)) return "t" + to_string(sym.base_index(v.base));
+        // A reduction's output that is a temporary of an outer loop is the schedule's accumulator too.
         auto ext = external_acc.find(ViewKey(v));
         if (ext != external_acc.end()) return ext->second;
+        if (s.is_tmp(v.base)) return "t" + to_string(sym.base_index(v.base));
         if (const string *r = s.replaced(v)) return *r;
         return array_ref(v, hidden_axis);
     }

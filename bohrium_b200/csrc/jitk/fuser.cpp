@@ -606,6 +606,39 @@ bool collapse_loop_with_child(LoopB &loop) {
 }
 } // namespace
 
+namespace {
+void forget_free(LoopB &loop, bh_base *base) {
+    loop._frees.erase(base);
+    for (Block &b : loop._block_list)
+        if (!b.isInstr()) forget_free(b.getLoop(), base);
+}
+
+// Loops that were taken apart carry their arrays' frees in every piece. Leave each with the last
+// block that accesses the array: freed with an earlier one, the array would be gone for the others,
+// or a register of that one.
+void settle_frees(vector<Block> &block_list, LoopB *parent = nullptr) {
+    map<const bh_base *, size_t> last;
+    for (size_t i = 0; i < block_list.size(); ++i) {
+        if (!block_list[i].isInstr()) settle_frees(block_list[i].getLoop()._block_list, &block_list[i].getLoop());
+        for (const bh_base *b : block_list[i].getAllBases()) last[b] = i;
+    }
+    for (size_t i = 0; i < block_list.size(); ++i) {
+        if (block_list[i].isInstr()) continue;
+        for (bh_base *b : block_list[i].getLoop().getAllFrees()) {
+            auto it = last.find(b);
+            if (it == last.end() || it->second == i) continue;
+            forget_free(block_list[i].getLoop(), b);
+            if (!block_list[it->second].isInstr()) {
+                LoopB &l = block_list[it->second].getLoop();
+                if (!l.getAllFrees().count(b)) l._frees.insert(b);
+            } else if (parent != nullptr) {
+                parent->_frees.insert(b);
+            }
+        }
+    }
+}
+} // namespace
+
 void push_reductions_inwards(vector<Block> &block_list) {
     vector<Block> list2(block_list);
     for (Block &b : list2)
@@ -772,8 +805,10 @@ vector<Block> fuse_block_list(const vector<bh_instruction *> &instr_list, const 
     for (const string &t : config.fuser_list) {
         if (t == "push_reductions_inwards") {
             push_reductions_inwards(block_list);
+            settle_frees(block_list);
         } else if (t == "split_for_threading") {
             split_for_threading(block_list);
+            settle_frees(block_list);
         } else if (t == "collapse_redundant_axes") {
             collapse_redundant_axes(block_list);
         } else if (t == "serial") {

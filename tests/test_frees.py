@@ -1,0 +1,73 @@
+"""Arrays that a flush frees while loops are taken apart (a reduction pushed inwards, loops split for
+threads): each is freed by the last kernel that reads or writes it, and is a register of no other."""
+import re
+
+import numpy as np
+import pytest
+
+import bohrium_b200 as bh
+
+
+def column_maximum_beside_row_values(x, r):
+    """The maxima over the rows run with the axes swapped, apart from the chain of row values."""
+    c = x.max(0)
+    u = r * 2 + 1
+    v = x * x
+    m = v - r.reshape(r.shape[0], 1)
+    return [c, m, u]
+
+
+def row_values_dropped_before_their_array(x, r):
+    u = r * 2 + 1
+    w = u * u
+    del u
+    c = x.max(0)
+    v = x + x
+    m = v - r.reshape(r.shape[0], 1)
+    del r
+    return [c, m, v, w]
+
+
+PROGRAMS = [column_maximum_beside_row_values, row_values_dropped_before_their_array]
+FUSERS = [None, "greedy,push_reductions_inwards,split_for_threading,collapse_redundant_axes"]
+
+
+@pytest.mark.parametrize("fusers", FUSERS)
+@pytest.mark.parametrize("prog", PROGRAMS, ids=lambda f: f.__name__)
+def test_frees_follow_the_last_access(prog, fusers):
+    rt = bh.Runtime(bh.DryRunExecutor())
+    x, r = bh.empty(rt, (2000, 31), np.int64), bh.empty(rt, (2000,), np.int64)
+    rt.flush()
+    keep = prog(x, r)
+    del r
+    blocks = [k["block"] for k in bh.dry_run(rt.take(), compile=False, fuser_list=fusers)["kernels"]]
+    assert len(keep) and len(blocks) > 1
+    freed = []
+    for i, block in enumerate(blocks):
+        here = {a for names in re.findall(r"frees: \{([^}]*)\}", block) for a in names.split(",") if a}
+        for a in here:
+            assert not any(re.search(rf"\b{a}\b", later) for later in blocks[i + 1:]), (a, blocks)
+        freed += here
+    assert len(freed) == len(set(freed)) > 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch", ["off", "grouped"])
+@pytest.mark.parametrize("prog", PROGRAMS, ids=lambda f: f.__name__)
+def test_values(gpu_executor, prog, batch):
+    rng = np.random.default_rng(0)
+    x, r = rng.integers(-9, 9, (200, 31)), rng.integers(-9, 9, 200)
+    gpu_executor.message("CUDA: batch " + batch)
+    try:
+        rt = bh.Runtime(gpu_executor)
+        for _ in range(3):  # other arrays have held other values by then
+            a, b = bh.array(rt, x), bh.array(rt, r)
+            rt.flush()
+            got = prog(a, b)
+            del b
+            rt.flush()
+            for g, w in zip(got, prog(x, r)):
+                np.testing.assert_array_equal(g.numpy(), w)
+            x, r = x + 1, r - 1
+    finally:
+        gpu_executor.message("CUDA: batch off")

@@ -8,8 +8,10 @@ import pytest
 import bohrium_b200 as bh
 
 
-def column_maximum_beside_row_values(x, r):
-    """The maxima over the rows run with the axes swapped, apart from the chain of row values."""
+def column_maximum_beside_row_values(args):
+    """The maxima over the rows run with the axes swapped, apart from the chain of row values. The
+    program holds the only references to its inputs, so they are freed too."""
+    x, r = args.pop(), args.pop()
     c = x.max(0)
     u = r * 2 + 1
     v = x * x
@@ -17,15 +19,14 @@ def column_maximum_beside_row_values(x, r):
     return [c, m, u]
 
 
-def row_values_dropped_before_their_array(x, r):
+def row_values_dropped_before_their_array(args):
+    x, r = args.pop(), args.pop()
     u = r * 2 + 1
-    w = u * u
     del u
     c = x.max(0)
-    v = x + x
+    v = np.maximum(x, x) if isinstance(x, np.ndarray) else bh.binary("MAXIMUM", x, x)
     m = v - r.reshape(r.shape[0], 1)
-    del r
-    return [c, m, v, w]
+    return [c, m, v]
 
 
 PROGRAMS = [column_maximum_beside_row_values, row_values_dropped_before_their_array]
@@ -36,10 +37,9 @@ FUSERS = [None, "greedy,push_reductions_inwards,split_for_threading,collapse_red
 @pytest.mark.parametrize("prog", PROGRAMS, ids=lambda f: f.__name__)
 def test_frees_follow_the_last_access(prog, fusers):
     rt = bh.Runtime(bh.DryRunExecutor())
-    x, r = bh.empty(rt, (2000, 31), np.int64), bh.empty(rt, (2000,), np.int64)
+    args = [bh.empty(rt, (200,), np.int64), bh.empty(rt, (200, 31), np.int64)]
     rt.flush()
-    keep = prog(x, r)
-    del r
+    keep = prog(args)
     blocks = [k["block"] for k in bh.dry_run(rt.take(), compile=False, fuser_list=fusers)["kernels"]]
     assert len(keep) and len(blocks) > 1
     freed = []
@@ -61,12 +61,11 @@ def test_values(gpu_executor, prog, batch):
     try:
         rt = bh.Runtime(gpu_executor)
         for _ in range(3):  # other arrays have held other values by then
-            a, b = bh.array(rt, x), bh.array(rt, r)
+            args = [bh.array(rt, r), bh.array(rt, x)]
             rt.flush()
-            got = prog(a, b)
-            del b
+            got = prog(args)
             rt.flush()
-            for g, w in zip(got, prog(x, r)):
+            for g, w in zip(got, prog([r, x])):
                 np.testing.assert_array_equal(g.numpy(), w)
             x, r = x + 1, r - 1
     finally:

@@ -9,6 +9,7 @@
 #include <cmath>
 #include <cstring>
 #include <functional>
+#include <list>
 #include <map>
 #include <regex>
 #include <set>
@@ -5222,6 +5223,20 @@ LaunchUnit fuse_tail(const LaunchUnit &u1, const LaunchUnit &u2) {
 constexpr int64_t kRowElements = 6;      // elements of a row per lane aimed at
 constexpr int64_t kRowElementsMost = 12; // and at most (with a whole CTA on a row)
 constexpr int kRowRegisters = 48;        // 4-byte registers of a row that a lane may carry between stages
+// A group's stages x its instructions over the row x the square of a lane's registers for one row
+// (elements x 4-byte words). The code of all stages is unrolled over a lane's elements, and the compiler
+// keeps more registers the more stages there are: past one CTA of 128 registers a thread on an SM, the
+// latency of the rows' chains shows. Kernels one by one against one unit, us: normalising a matrix by its
+// row sums 4, 8 and 16 times over (5, 9 and 17 stages of 2 instructions), float64 8000 x 3072 (12 elements, 24
+// words) 310 -> 211, 577 -> 715, 1114 -> 1790, float64 20000 x 1500 (12 words) 389 -> 229, 747 -> 533, 1461 -> 1896,
+// float32 20000 x 1500 (6 words) 250 -> 120, 455 -> 235, 865 -> 749; two softmaxes of one matrix (5 stages, 11
+// instructions) 334 -> 269 at 24 words, four (9, 21) 662 -> 904 there, 861 -> 602 at 12 and 488 -> 216 at 6;
+// 20 instructions in 5 stages 377 -> 594 at 24 words, 493 -> 484 at 12 and 273 -> 172 at 6.
+constexpr int64_t kRowCost = 33000;
+// Stages of a group, where rows are short: 17 in one unit took 181 us and in units of 6 and of 8 113 and 120
+// us (float32 20000 x 300), 9 in one unit 51 us and in units of 6 and 3 58 us.
+constexpr size_t kRowStagesMost = 9;
+constexpr int64_t kRowUnrolledMost = 1024; // instructions over the row x elements of a lane: code written out
 
 struct RowStage {
     const LoopB *loop = nullptr; // the rank-0 loop
@@ -5258,9 +5273,15 @@ bool row_stage(const LoopB &kernel, const vector<LaunchUnit> &units, RowStage &s
     return loops == 1;
 }
 
-// Lowers `stages` (the kernels' loops, in order) as one unit; false when they are not row-local or
-// too large. `unseen`: arrays that nothing outside the group sees.
-bool lower_rows(const vector<RowStage> &stages, const set<const bh_base *> &unseen, const CodegenOptions &opt, LaunchUnit &u) {
+// Whether stages can run as one unit: never (they are not row-local, or too large: more stages do
+// not change that), not yet (nothing they share would stay in registers, or no reduction among them),
+// or as they are.
+enum class RowFit { NEVER, NOT_YET, FITS };
+
+// Lowers `stages` (the kernels' loops, in order) as one unit, or only tells whether they fit (no `u`).
+// `unseen`: arrays that nothing outside the group sees.
+RowFit lower_rows(const vector<RowStage> &stages, const set<const bh_base *> &unseen, const CodegenOptions &opt, LaunchUnit *out) {
+    if (stages.size() > kRowStagesMost) return RowFit::NEVER;
     const int64_t points = stages[0].loop->size, len = stages[0].sub->size;
     vector<Block> holders;
     holders.reserve(stages.size());
@@ -5295,6 +5316,7 @@ bool lower_rows(const vector<RowStage> &stages, const set<const bh_base *> &unse
     };
     vector<Use> uses;
     set<const bh_base *> written;
+    int64_t row_instrs = 0;  // instructions over the row
     for (size_t i = 0; i < st.size(); ++i) {
         vector<pair<InstrPtr, bool>> instrs;
         for (const InstrPtr &ip : jitk::all_instr(*st[i].sub)) instrs.emplace_back(ip, true);
@@ -5308,9 +5330,10 @@ bool lower_rows(const vector<RowStage> &stages, const set<const bh_base *> &unse
         for (const auto &pi : instrs) {
             const bh_instruction &in = *pi.first;
             if (bh_opcode_is_system(in.opcode) || in.operand.empty()) continue;
+            row_instrs += pi.second ? 1 : 0;
             if (in.opcode == BH_GATHER || in.opcode == BH_SCATTER || in.opcode == BH_COND_SCATTER ||
                 bh_opcode_is_accumulate(in.opcode))
-                return false;
+                return RowFit::NEVER;
             for (size_t o = 1; o < in.operand.size(); ++o)
                 if (!in.operand[o].isConstant()) uses.push_back({i, &in.operand[o], false, pi.second});
             uses.push_back({i, &in.operand[0], true, pi.second});
@@ -5337,12 +5360,12 @@ bool lower_rows(const vector<RowStage> &stages, const set<const bh_base *> &unse
             // a reduction's output and what follows it are one value per row
             const bool scalar = !two;
             if (scalar) {
-                if (v.ndim != 1 || v.stride[0] == 0 || row_of.count(b)) return false;
+                if (v.ndim != 1 || v.stride[0] == 0 || row_of.count(b)) return RowFit::NEVER;
                 const auto at = make_pair(v.start, v.stride[0]);
                 auto it = scalars.emplace(b, at).first;
-                if (it->second != at) return false;
+                if (it->second != at) return RowFit::NEVER;
             } else {
-                if (scalars.count(b) || v.stride[1] == 0 || abs(v.stride[0]) < (len - 1) * abs(v.stride[1]) + 1) return false;
+                if (scalars.count(b) || v.stride[1] == 0 || abs(v.stride[0]) < (len - 1) * abs(v.stride[1]) + 1) return RowFit::NEVER;
                 row_of.emplace(b, &v);
             }
         }
@@ -5355,14 +5378,14 @@ bool lower_rows(const vector<RowStage> &stages, const set<const bh_base *> &unse
         if (sc != scalars.end()) {
             const bool same = v.start == sc->second.first && v.ndim >= 1 && v.stride[0] == sc->second.second &&
                               (v.ndim == 1 || (v.ndim == 2 && v.stride[1] == 0));
-            if (!same) return false;
+            if (!same) return RowFit::NEVER;
             // a per-row value must be there before it is read: written by an earlier stage or instruction
             continue;
         }
         auto ro = row_of.find(b);
-        if (ro != row_of.end() && !(v == *ro->second)) return false;
+        if (ro != row_of.end() && !(v == *ro->second)) return RowFit::NEVER;
         if (!x.in_row) {
-            if (ro != row_of.end()) return false;
+            if (ro != row_of.end()) return RowFit::NEVER;
             continue;  // a 1-D array read after a reduction
         }
         if (v.ndim != 2 || v.stride[1] == 0) continue;  // read from memory where it is used
@@ -5383,7 +5406,7 @@ bool lower_rows(const vector<RowStage> &stages, const set<const bh_base *> &unse
         for (const Use &x : uses) {
             if (!scalars.count(x.v->base)) continue;
             if (x.write) seen.insert(x.v->base);
-            else if (!seen.count(x.v->base)) return false;
+            else if (!seen.count(x.v->base)) return RowFit::NEVER;
         }
     }
     // What one stage alone touches is read and written in memory; the others live in registers from
@@ -5392,17 +5415,23 @@ bool lower_rows(const vector<RowStage> &stages, const set<const bh_base *> &unse
     rows.erase(remove_if(rows.begin(), rows.end(), [&](const RowArray &r) { return r.first == r.last && !dropped.count(r.view.base); }),
                rows.end());
     int live = 0;
+    int64_t word = 1;  // 4-byte registers of an element
+    for (const RowArray &r : rows) word = max<int64_t>(word, (bh_type_size(r.view.base->dtype()) + 3) / 4);
     for (size_t i = 0; i + 1 < st.size(); ++i) {
         int words = 0;
         for (const RowArray &r : rows)
             if (r.first <= i && i < r.last) words += (static_cast<int>(bh_type_size(r.view.base->dtype())) + 3) / 4;
         live = max(live, words);
     }
-    if (live == 0) return false;
     int64_t C = lane_count(points, len);
     while (C < kThreads && (len + C - 1) / C > kRowElements) C *= 2;
     const int64_t NU = (len + C - 1) / C;
-    if (C < 2 || NU > kRowElementsMost || NU * live > kRowRegisters) return false;
+    if (C < 2 || NU > kRowElementsMost || NU * live > kRowRegisters || NU * row_instrs > kRowUnrolledMost ||
+        static_cast<int64_t>(st.size()) * row_instrs * (NU * word) * (NU * word) > kRowCost)
+        return RowFit::NEVER;
+    if (live == 0 || none_of(st.begin(), st.end(), [](const RowStage &x) { return x.reduce; })) return RowFit::NOT_YET;
+    if (out == nullptr) return RowFit::FITS;
+    LaunchUnit &u = *out;
     for (const bh_base *b : dropped) sym.temps.insert(b);
     // Rebuild the parameters without the dropped arrays.
     {
@@ -5491,18 +5520,24 @@ bool lower_rows(const vector<RowStage> &stages, const set<const bh_base *> &unse
         body << "        const int i1 = lane + u * " << C << ";\n";
         body << "        if (i1 < n) {\n" << inside << "        }\n    }\n";
     };
-    {
+    // A row array that is read before it is written is loaded where its first stage begins: no
+    // register holds it before.
+    auto emit_loads = [&](size_t stage) {
         string loads;
         for (size_t k = 0; k < rows.size(); ++k)
-            if (rows[k].load) loads += "            ra" + to_string(k) + "[u] = " + row_ref(k) + ";\n";
+            if (rows[k].load && rows[k].first == stage) loads += "            ra" + to_string(k) + "[u] = " + row_ref(k) + ";\n";
         if (!loads.empty()) unrolled(loads);
-    }
+    };
     // Values per row: reduction results and what instructions after a reduction make of them.
     map<const bh_base *, string> value;
-    for (const auto &sc : scalars) {
-        const string nm = "rv" + to_string(sym.base_index(sc.first));
-        value[sc.first] = nm;
-        body << "    " << cuda_type(sc.first->dtype()) << " " << nm << ";\n";
+    vector<const bh_base *> row_values;  // in the order of their first use, not of their addresses
+    for (const auto &sc : scalars) row_values.push_back(sc.first);
+    sort(row_values.begin(), row_values.end(),
+         [&](const bh_base *a, const bh_base *b) { return sym.base_index(a) < sym.base_index(b); });
+    for (const bh_base *b : row_values) {
+        const string nm = "rv" + to_string(sym.base_index(b));
+        value[b] = nm;
+        body << "    " << cuda_type(b->dtype()) << " " << nm << ";\n";
     }
     for (const Use &x : uses)
         if (value.count(x.v->base)) g.repl[ViewKey(*x.v)] = value.at(x.v->base);
@@ -5510,6 +5545,7 @@ bool lower_rows(const vector<RowStage> &stages, const set<const bh_base *> &unse
     for (size_t i = 0; i < st.size(); ++i) {
         Scope s;
         s.parent = &g;
+        emit_loads(i);
         body << "    {\n";
         for (Red &r : reds[i]) {
             body << "    " << r.T << " " << r.acc << " = " << r.ident << ";\n";
@@ -5567,11 +5603,11 @@ bool lower_rows(const vector<RowStage> &stages, const set<const bh_base *> &unse
         body << "    }\n";
     }
     string stores;
-    for (const auto &sc : scalars) {
-        if (dropped.count(sc.first)) continue;
+    for (const bh_base *b : row_values) {
+        if (dropped.count(b)) continue;
         for (const Use &x : uses)
-            if (x.write && x.v->base == sc.first) {
-                stores += "        " + em.array_ref(*x.v, x.in_row ? 1 : BH_MAXDIM) + " = " + value.at(sc.first) + ";\n";
+            if (x.write && x.v->base == b) {
+                stores += "        " + em.array_ref(*x.v, x.in_row ? 1 : BH_MAXDIM) + " = " + value.at(b) + ";\n";
                 break;
             }
     }
@@ -5581,72 +5617,241 @@ bool lower_rows(const vector<RowStage> &stages, const set<const bh_base *> &unse
     u.algorithmic_bytes = unit_bytes(sym, items);
     u.elements = points * len;
     finish_source(u, pl.decl.str(), body.str(), opt);
-    return true;
+    return RowFit::FITS;
 }
 
-// Row fusion over a flush's lowered kernels: the first kernel of each group gets the group's unit,
-// the others' unit lists are emptied and `into` names the first.
+// The part of a row stage's rank-0 loop whose instructions `keep` and whose arrays' frees `frees` names.
+LoopB part_of_loop(const LoopB &loop, const function<bool(const InstrPtr &)> &keep, const function<bool(const bh_base *)> &frees) {
+    LoopB part = loop;
+    part._block_list.clear();
+    for (const Block &b : loop._block_list) {
+        if (b.isInstr()) {
+            if (keep(b.getInstr())) part._block_list.push_back(b);
+        } else {
+            LoopB sub = part_of_loop(b.getLoop(), keep, frees);
+            if (!sub._block_list.empty()) part._block_list.emplace_back(std::move(sub));
+        }
+    }
+    part._frees.clear();
+    for (bh_base *b : loop._frees)
+        if (frees(b)) part._frees.insert(b);
+    part.metadataUpdate();
+    return part;
+}
+
+// Row fusion over a run of neighbouring kernels that are row stages of one index space. The fuser
+// merges independent work of one shape into one kernel (the last map of a softmax with the first
+// maximum of the next one), so the groups are made of instructions, not of kernels: those that share
+// a row array, an array that the run writes or one that it frees belong together, and what shares
+// none of these is apart, and its kernels are taken apart for it. Each group's stages then run as the
+// longest sequences that fit one unit (lower_rows). Kernels that share groups run at the first of
+// them; groups have nothing to wait for in one another.
+void fuse_row_run(const vector<LoopB> &kernels, const vector<size_t> &run, const vector<RowStage> &stages,
+                  const map<const bh_base *, set<size_t>> &touches, const set<const bh_base *> &transient,
+                  vector<vector<LaunchUnit>> &lowered, const CodegenOptions &opt, vector<int> &into) {
+    // Groups of instructions, by a union of their arrays.
+    struct Node {
+        size_t kernel;  // index in `run`
+        InstrPtr instr;
+        bool in_row;    // over the row, not after a reduction
+    };
+    vector<Node> nodes;
+    vector<size_t> first_node;  // of each kernel
+    set<const bh_base *> joins;
+    for (size_t m = 0; m < run.size(); ++m) {
+        first_node.push_back(nodes.size());
+        for (const InstrPtr &ip : jitk::all_instr(*stages[m].loop)) {
+            if (bh_opcode_is_system(ip->opcode) || ip->operand.empty()) continue;
+            const bool local = [&] {
+                for (const Block &b : stages[m].loop->_block_list)
+                    if (b.isInstr() && b.getInstr() == ip) return true;
+                return false;
+            }();
+            nodes.push_back({m, ip, !local});
+            if (!ip->operand[0].isConstant()) joins.insert(ip->operand[0].base);
+            for (const bh_view &v : ip->operand)
+                if (!v.isConstant() && v.ndim == 2 && v.stride[1] != 0) joins.insert(v.base);
+        }
+        for (const bh_base *f : kernels[run[m]].getAllFrees()) joins.insert(f);
+    }
+    first_node.push_back(nodes.size());
+    vector<size_t> parent(nodes.size());
+    for (size_t i = 0; i < parent.size(); ++i) parent[i] = i;
+    function<size_t(size_t)> root = [&](size_t i) { return parent[i] == i ? i : parent[i] = root(parent[i]); };
+    map<const bh_base *, size_t> holder;  // a node of each joining array
+    for (size_t i = 0; i < nodes.size(); ++i)
+        for (const bh_view &v : nodes[i].instr->operand)
+            if (!v.isConstant() && joins.count(v.base)) parent[root(i)] = root(holder.emplace(v.base, i).first->second);
+    // Instructions after a kernel's reductions stay with one of them.
+    for (size_t i = 0; i < nodes.size(); ++i) {
+        if (nodes[i].in_row) continue;
+        size_t sweep = nodes.size();
+        bool with_one = false;
+        for (size_t j = first_node[nodes[i].kernel]; j < first_node[nodes[i].kernel + 1]; ++j) {
+            if (!nodes[j].in_row || !bh_opcode_is_sweep(nodes[j].instr->opcode)) continue;
+            sweep = min(sweep, j);
+            with_one = with_one || root(j) == root(i);
+        }
+        if (sweep == nodes.size()) return;
+        if (!with_one) parent[root(i)] = root(sweep);
+    }
+    struct Member {
+        size_t kernel;  // index in `run`
+        RowStage stage;
+        bool whole;     // all of the kernel
+    };
+    map<size_t, vector<Member>> groups;           // by root
+    vector<size_t> order;                         // roots, by their first instruction
+    vector<set<size_t>> of_kernel(run.size());    // groups of each kernel
+    for (size_t i = 0; i < nodes.size(); ++i) {
+        if (groups.emplace(root(i), vector<Member>()).second) order.push_back(root(i));
+        of_kernel[nodes[i].kernel].insert(root(i));
+    }
+    list<LoopB> parts;
+    for (size_t m = 0; m < run.size(); ++m)
+        for (size_t g : of_kernel[m]) {
+            Member x{m, stages[m], of_kernel[m].size() == 1};
+            if (!x.whole) {
+                set<const bh_instruction *> mine;
+                for (size_t i = first_node[m]; i < first_node[m + 1]; ++i)
+                    if (root(i) == g) mine.insert(nodes[i].instr.get());
+                parts.push_back(part_of_loop(
+                    *stages[m].loop, [&](const InstrPtr &ip) { return mine.count(ip.get()) > 0; },
+                    [&](const bh_base *b) {
+                        auto h = holder.find(b);
+                        return h != holder.end() && root(h->second) == g;
+                    }));
+                x.stage.loop = &parts.back();
+                x.stage.sub = nullptr;
+                for (const Block &b : parts.back()._block_list)
+                    if (!b.isInstr() && !b.isSystemOnly()) x.stage.sub = &b.getLoop();
+                if (x.stage.sub == nullptr) return;
+                x.stage.reduce = !x.stage.sub->_sweeps.empty();
+            }
+            groups.at(g).push_back(x);
+        }
+    map<size_t, vector<const bh_base *>> passing;  // transient arrays of each group
+    for (const bh_base *b : transient) {
+        auto h = holder.find(b);
+        if (h != holder.end()) passing[root(h->second)].push_back(b);
+    }
+    // The groups' units.
+    struct Made {
+        bool fused = false;
+        vector<LaunchUnit> units;
+    };
+    map<size_t, Made> made;
+    for (size_t g : order) {
+        const vector<Member> &ms = groups.at(g);
+        Made &r = made[g];
+        for (size_t i = 0; i < ms.size();) {
+            vector<RowStage> seq, best;
+            set<size_t> in;
+            set<const bh_base *> unseen, best_unseen;
+            for (size_t j = i; j < ms.size(); ++j) {
+                seq.push_back(ms[j].stage);
+                in.insert(run[ms[j].kernel]);
+                unseen.clear();
+                for (const bh_base *b : passing[g]) {
+                    const set<size_t> &t = touches.at(b);
+                    if (all_of(t.begin(), t.end(), [&](size_t k) { return in.count(k) > 0; })) unseen.insert(b);
+                }
+                const RowFit fit = j == i ? RowFit::NOT_YET : lower_rows(seq, unseen, opt, nullptr);
+                if (fit == RowFit::NEVER) break;
+                if (fit == RowFit::FITS) {
+                    best = seq;
+                    best_unseen = unseen;
+                }
+            }
+            LaunchUnit u;
+            bool fused = false;
+            try {
+                fused = !best.empty() && lower_rows(best, best_unseen, opt, &u) == RowFit::FITS;
+            } catch (const out_of_range &) {
+                // an operand that the unit has neither in registers nor among its arrays: the
+                // kernels run one by one
+            }
+            if (fused) {
+                r.units.push_back(std::move(u));
+                r.fused = true;
+                i += best.size();
+                continue;
+            }
+            if (ms[i].whole) {
+                r.units.push_back(lowered[run[ms[i].kernel]][0]);
+            } else {
+                LoopB kernel{-1, 1};
+                kernel._block_list.emplace_back(*ms[i].stage.loop);
+                kernel.metadataUpdate();
+                for (LaunchUnit &x : lower_kernel(kernel, opt)) r.units.push_back(std::move(x));
+            }
+            ++i;
+        }
+    }
+    // Kernels that share groups, and have a fused one among them, run at the first of them.
+    vector<bool> done(run.size(), false);
+    for (size_t m = 0; m < run.size(); ++m) {
+        if (done[m]) continue;
+        set<size_t> gs = of_kernel[m], ks{m};
+        for (bool grown = true; grown;) {
+            grown = false;
+            for (size_t k = 0; k < run.size(); ++k) {
+                if (ks.count(k) || none_of(of_kernel[k].begin(), of_kernel[k].end(), [&](size_t g) { return gs.count(g) > 0; })) continue;
+                ks.insert(k);
+                gs.insert(of_kernel[k].begin(), of_kernel[k].end());
+                grown = true;
+            }
+        }
+        for (size_t k : ks) done[k] = true;
+        if (none_of(gs.begin(), gs.end(), [&](size_t g) { return made.at(g).fused; })) continue;
+        vector<LaunchUnit> units;
+        for (size_t g : order) {
+            if (!gs.count(g)) continue;
+            int step = 0;
+            for (LaunchUnit &u : made.at(g).units) {
+                u.step = step++;
+                units.push_back(std::move(u));
+            }
+        }
+        for (size_t k : ks) {
+            lowered[run[k]].clear();
+            if (k != m) into[run[k]] = static_cast<int>(run[m]);
+        }
+        lowered[run[m]] = std::move(units);
+    }
+}
+
+// Row fusion over a flush's lowered kernels: the first kernel of a group gets its units, the others'
+// unit lists are emptied and `into` names the first.
 void fuse_rows(const vector<LoopB> &kernels, vector<vector<LaunchUnit>> &lowered, const CodegenOptions &opt, vector<int> &into) {
     const size_t n = kernels.size();
     // Kernels that touch each array, and arrays created and freed by the flush.
     map<const bh_base *, set<size_t>> touches;
-    set<const bh_base *> created, freed;
-    for (size_t k = 0; k < n; ++k) {
+    set<const bh_base *> created, transient;
+    for (size_t k = 0; k < n; ++k)
         for (const InstrPtr &ip : jitk::all_instr(kernels[k])) {
             if (bh_opcode_is_system(ip->opcode)) continue;
             for (size_t o = 0; o < ip->operand.size(); ++o)
                 if (!ip->operand[o].isConstant()) touches[ip->operand[o].base].insert(k);
             if (ip->constructor && !ip->operand.empty() && !ip->operand[0].isConstant()) created.insert(ip->operand[0].base);
         }
-        for (const bh_base *f : kernels[k].getAllFrees()) freed.insert(f);
-    }
+    for (size_t k = 0; k < n; ++k)
+        for (const bh_base *f : kernels[k].getAllFrees())
+            if (created.count(f)) transient.insert(f);
     for (size_t k = 0; k < n; ++k) {
-        RowStage first;
-        if (lowered[k].empty() || !row_stage(kernels[k], lowered[k], first) || first.loop->size < kLaneMinPoints) continue;
-        vector<RowStage> group{first};
-        vector<size_t> members{k};
-        LaunchUnit best;
-        bool have = false;
-        size_t used = 1;
-        bool any_reduce = first.reduce;
-        for (size_t j = k + 1; j < n; ++j) {
+        vector<size_t> run;
+        vector<RowStage> stages;
+        size_t j = k;
+        for (; j < n; ++j) {
             if (kernels[j].isSystemOnly()) continue;
             RowStage next;
-            if (!row_stage(kernels[j], lowered[j], next) || next.loop->size != first.loop->size ||
-                next.sub->size != first.sub->size)
-                break;
-            group.push_back(next);
-            members.push_back(j);
-            any_reduce = any_reduce || next.reduce;
-            if (!any_reduce) continue;
-            const set<size_t> in(members.begin(), members.end());
-            set<const bh_base *> unseen;
-            for (const auto &t : touches) {
-                if (!created.count(t.first) || !freed.count(t.first)) continue;
-                bool inside = true;
-                for (size_t m : t.second) inside = inside && in.count(m);
-                if (inside) unseen.insert(t.first);
-            }
-            // something has to be shared: a row array two of the kernels touch
-            bool shared = false;
-            for (const auto &t : touches) {
-                int c = 0;
-                for (size_t m : t.second) c += in.count(m) ? 1 : 0;
-                shared = shared || (c > 1 && t.first->nelem() >= first.loop->size * first.sub->size);
-            }
-            LaunchUnit u;
-            if (shared && lower_rows(group, unseen, opt, u)) {
-                best = std::move(u);
-                have = true;
-                used = group.size();
-            }
+            if (lowered[j].empty() || !row_stage(kernels[j], lowered[j], next) || next.loop->size < kLaneMinPoints) break;
+            if (!stages.empty() && (next.loop->size != stages[0].loop->size || next.sub->size != stages[0].sub->size)) break;
+            run.push_back(j);
+            stages.push_back(next);
         }
-        if (!have) continue;
-        lowered[k].assign(1, best);
-        for (size_t m = 1; m < used; ++m) {
-            lowered[members[m]].clear();
-            into[members[m]] = static_cast<int>(k);
-        }
+        if (run.size() > 1) fuse_row_run(kernels, run, stages, touches, transient, lowered, opt, into);
+        if (!run.empty()) k = run.back();
     }
 }
 
@@ -5805,6 +6010,7 @@ vector<int> fuse_tails(const vector<LoopB> &kernels, vector<vector<LaunchUnit>> 
         for (size_t m = k + 1; m < j && commutes; ++m)
             commutes = !meets(writes[m], reads[j]) && !meets(writes[m], writes[j]) && !meets(reads[m], writes[j]);
         if (!commutes || lowered[k].empty() || into[k] >= 0) continue;
+        if (lowered[k].size() > 1 && lowered[k].back().step >= 0) continue;  // units that run side by side
         LaunchUnit &u1 = lowered[k].back();
         if (u1.tail || u1.sched == Sched::SCAN1D || u1.sched == Sched::AXIS_SCAN || u1.sched == Sched::SERIAL || u1.sched == Sched::TILE2D ||
             u1.body_core.empty())

@@ -150,6 +150,9 @@ struct LaunchUnit {
     // This unit's kernel runs a folded reduction's bh_tail in the CTA that finishes last; the
     // completion counter follows the unit's own counters.
     bool tail = false;
+    // Its place among its kernel's units: it runs after those of smaller steps (row groups of one
+    // kernel have equal steps and do not wait for one another). Negative: its index in the list.
+    int step = -1;
     int64_t work_items() const;
     int64_t grouped_work_items() const; // work items when launched grouped (batch_chunks)
     int64_t scratch_bytes() const;   // partials in the scratch arena

@@ -1355,6 +1355,8 @@ EngineCUDA::FlushPlan EngineCUDA::build_plan(const vector<LoopB> &kernels, const
                 for (size_t f = 0; f < u.fields.size(); ++f)
                     if (u.fields[f].kind == ParamField::PTR || u.fields[f].kind == ParamField::TMAP)
                         pu.ptr_base[f] = idx(u.fields[f].base);
+                pu.step = u.step >= 0 ? u.step : static_cast<int>(pk.units.size());
+                pk.depth = max(pk.depth, pu.step + 1);
                 pu.unit = std::move(u);
                 pk.units.push_back(std::move(pu));
             }
@@ -1408,7 +1410,7 @@ EngineCUDA::FlushPlan EngineCUDA::build_plan(const vector<LoopB> &kernels, const
         for (int b : reads) level = max(level, last_write_level[b] + 1);
         for (int b : writes) level = max(level, max(last_write_level[b], last_read_level[b]) + 1);
         pk.level = level;
-        const int end_level = level + max<int>(static_cast<int>(pk.units.size()), 1) - 1;
+        const int end_level = level + pk.depth - 1;
         for (int b : reads) last_read_level[b] = max(last_read_level[b], end_level);
         for (int b : writes) last_write_level[b] = max(last_write_level[b], end_level);
         plan.nlevels = max(plan.nlevels, end_level + 1);
@@ -1427,7 +1429,7 @@ void EngineCUDA::run_plan(const FlushPlan &plan, const vector<bh_base *> &bases,
     // A replay whose writes are all still in host_stale (nothing was removed from it since its
     // last run) need not insert them again.
     const bool stale_known = replay != nullptr && replay->stale_after == stale_epoch;
-    if (batch_mode == "off" || plan.kernels.size() < 2) {
+    if (batch_mode == "off" || plan.one_by_one()) {
         for (const PlanKernel &pk : plan.kernels) {
             ++_stats.kernels;
             for (const PlanUnit &pu : pk.units) launch_plain(pu, bases, instrs);
@@ -1443,8 +1445,8 @@ void EngineCUDA::run_plan(const FlushPlan &plan, const vector<bh_base *> &bases,
     vector<vector<const PlanKernel *>> kernels_by_end(static_cast<size_t>(plan.nlevels));
     for (const PlanKernel &pk : plan.kernels) {
         ++_stats.kernels;
-        for (size_t j = 0; j < pk.units.size(); ++j) by_level[pk.level + j].push_back(&pk.units[j]);
-        kernels_by_end[pk.level + max<size_t>(pk.units.size(), 1) - 1].push_back(&pk);
+        for (const PlanUnit &pu : pk.units) by_level[static_cast<size_t>(pk.level + pu.step)].push_back(&pu);
+        kernels_by_end[static_cast<size_t>(pk.level + pk.depth - 1)].push_back(&pk);
     }
     for (size_t lv = 0; lv < by_level.size(); ++lv) {
         map<const Compiled *, vector<const PlanUnit *>> groups;

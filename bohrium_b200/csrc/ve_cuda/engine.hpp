@@ -261,12 +261,14 @@ private:
         LaunchUnit unit;
         Compiled *compiled = nullptr;
         std::vector<int> ptr_base; // per field: index of the base in flush order (PTR fields)
+        int step = 0;              // levels after the kernel's first unit
     };
     struct PlanKernel {
         std::vector<PlanUnit> units;
         std::vector<int> frees, writes;
         int level = 0; // dependency level of the first unit
-        jitk::CostFeatures feat{}; // cost-model features (when recording or learning)
+        int depth = 1; // levels of its units
+        jitk::CostFeatures feat{}; // cost-model features (when recording)
     };
     struct FlushPlan {
         std::vector<PlanKernel> kernels;
@@ -276,6 +278,10 @@ private:
         std::map<int64_t, std::string> orders;
         int64_t scan_bytes = 0; // scan arena the plan's SCAN1D units need
         std::string signature() const; // kernel names by level (plans with equal signatures match)
+        // No two units can share a launch.
+        bool one_by_one() const {
+            return kernels.empty() || (kernels.size() == 1 && kernels[0].depth >= static_cast<int>(kernels[0].units.size()));
+        }
     };
     std::unordered_map<uint64_t, FlushPlan> plans;
     // Replay of a fingerprinted BhIR (BhIRHints::fingerprint): the plan, the bases in flush order,

@@ -113,13 +113,13 @@ bool EngineCUDA::build_graph(Replay &r) {
 
     // The launches, grouped as run_plan groups them in "grouped" mode.
     vector<vector<const PlanUnit *>> launches;  // each entry: one plain unit or one group
-    if (plan.kernels.size() < 2) {
+    if (plan.one_by_one()) {
         for (const PlanKernel &pk : plan.kernels)
             for (const PlanUnit &pu : pk.units) launches.push_back({&pu});
     } else {
         vector<vector<const PlanUnit *>> by_level(static_cast<size_t>(plan.nlevels));
         for (const PlanKernel &pk : plan.kernels)
-            for (size_t j = 0; j < pk.units.size(); ++j) by_level[static_cast<size_t>(pk.level) + j].push_back(&pk.units[j]);
+            for (const PlanUnit &pu : pk.units) by_level[static_cast<size_t>(pk.level + pu.step)].push_back(&pu);
         for (const auto &level : by_level) {
             map<const Compiled *, vector<const PlanUnit *>> groups;
             vector<const Compiled *> order;

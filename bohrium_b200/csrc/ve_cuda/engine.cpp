@@ -163,6 +163,7 @@ EngineCUDA::EngineCUDA(component::ComponentVE &c) : comp(c) {
     ensure_counters(4096);
     check(cudaMalloc(&err_record, sizeof(unsigned long long)), "cudaMalloc(err)");
     check(cudaMemset(err_record, 0, sizeof(unsigned long long)), "cudaMemset(err)");
+    if (noalloc_sum_set_up(_device, _stream) != 0) throw runtime_error(bhb_last_error());
     if (!cache_dir.empty()) mkdir(cache_dir.c_str(), 0755);
     autotune = cfg.defaultGet<bool>("autotune", true);
     tune_min_elements = cfg.defaultGet<int64_t>("autotune_min_elements", 1 << 20);

@@ -30,6 +30,10 @@ struct bh_costmodel; // the cost model's network (mlp.cu)
 namespace bohrium {
 namespace cuda {
 
+// Set-up of bh_ve_cuda_sum_f64_noalloc on a device, so that its first call there allocates nothing
+// either (noalloc_sum.cu). `stream` is waited for. Returns 0, or -1 with bhb_last_error() set.
+int noalloc_sum_set_up(int device, void *stream);
+
 struct DeviceApi; // driver entry points (engine.cpp)
 
 // Per-launch-unit timing record (device time measured with CUDA events when profiling).

@@ -40,7 +40,8 @@ constexpr int kMaxDevices = 64;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
-// Per-device set-up, filled by the first call on each device. `scratch` is published with release
+// Per-device set-up, filled when an engine is created on a device or else by the first call there.
+// `scratch` is published with release
 // order after `max_ctas` is written, so a thread that reads a non-null `scratch` (acquire) also
 // sees `max_ctas`; concurrent first calls on one device serialise on g_setup_mutex.
 struct DeviceSetup {
@@ -122,7 +123,52 @@ int fail(const char *what, cudaError_t e) {
     return -1;
 }
 
+// Set-up, once per device, with that device current: the device address of the static scratch array
+// and the persistent grid size. With `warm` (a stream that is not being captured) the driver's own
+// first-use work happens here too: loading a module, its kernel or the memset's can take a block of
+// device memory, which no call may do later. One element of the scratch is summed into another, before
+// any other thread can see the array.
+int set_up(int dev, const cudaStream_t *warm) {
+    DeviceSetup &ds = g_setup[dev];
+    std::lock_guard<std::mutex> lock(g_setup_mutex);
+    if (ds.scratch.load(std::memory_order_acquire) != nullptr) return 0;
+    void *ptr = nullptr;
+    cudaError_t e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch);
+    if (e != cudaSuccess) return fail("cudaGetSymbolAddress", e);
+    int sms = 0, occ = 0;
+    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return fail("cudaDeviceGetAttribute", e);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, noalloc_sum_kernel, kThreads, 0);
+    if (e != cudaSuccess) return fail("cudaOccupancyMaxActiveBlocksPerMultiprocessor", e);
+    unsigned char *scratch = static_cast<unsigned char *>(ptr);
+    if (warm != nullptr) {
+        double *cells = reinterpret_cast<double *>(scratch);
+        e = cudaMemsetAsync(scratch + kCounterOffset, 0, sizeof(unsigned int), *warm);
+        if (e == cudaSuccess) {
+            noalloc_sum_kernel<<<1, kThreads, 0, *warm>>>(cells + 1, 1, cells + 2, scratch);
+            e = cudaGetLastError();
+        }
+        if (e == cudaSuccess) e = cudaStreamSynchronize(*warm);
+        if (e != cudaSuccess) return fail("set-up", e);
+    }
+    ds.max_ctas = static_cast<int64_t>(sms) * (occ > 0 ? occ : 1);
+    ds.scratch.store(scratch, std::memory_order_release);
+    return 0;
+}
+
 } // namespace
+
+namespace bohrium {
+namespace cuda {
+
+// Called when an engine is created, with its device current.
+int noalloc_sum_set_up(int device, void *stream) {
+    const cudaStream_t s = static_cast<cudaStream_t>(stream);
+    return device < 0 || device >= kMaxDevices ? 0 : set_up(device, &s);
+}
+
+} // namespace cuda
+} // namespace bohrium
 
 // Declared in include/bh_b200.h. Returns 0 on success, -1 with bhb_last_error() set on error.
 extern "C" int bh_ve_cuda_sum_f64_noalloc(const double *in, int64_t n, double *out, void *stream) {
@@ -148,27 +194,12 @@ extern "C" int bh_ve_cuda_sum_f64_noalloc(const double *in, int64_t n, double *o
         bhb_set_last_error("bh_ve_cuda_sum_f64_noalloc: device ordinal out of range");
         return -1;
     }
-    // Set-up, once per device, with that device current: the device address of the static
-    // scratch array and the persistent grid size. The first call on a device should come before
-    // any stream capture on it.
+    // The first call on a device where no engine was created should come before any stream capture on it.
     DeviceSetup &ds = g_setup[dev];
     unsigned char *scratch = ds.scratch.load(std::memory_order_acquire);
     if (scratch == nullptr) {
-        std::lock_guard<std::mutex> lock(g_setup_mutex);
+        if (set_up(dev, nullptr) != 0) return -1;
         scratch = ds.scratch.load(std::memory_order_acquire);
-        if (scratch == nullptr) {
-            void *ptr = nullptr;
-            e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch);
-            if (e != cudaSuccess) return fail("cudaGetSymbolAddress", e);
-            int sms = 0, occ = 0;
-            e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            if (e != cudaSuccess) return fail("cudaDeviceGetAttribute", e);
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, noalloc_sum_kernel, kThreads, 0);
-            if (e != cudaSuccess) return fail("cudaOccupancyMaxActiveBlocksPerMultiprocessor", e);
-            ds.max_ctas = static_cast<int64_t>(sms) * (occ > 0 ? occ : 1);
-            scratch = static_cast<unsigned char *>(ptr);
-            ds.scratch.store(scratch, std::memory_order_release);
-        }
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     e = cudaMemsetAsync(scratch + kCounterOffset, 0, sizeof(unsigned int), s);

@@ -1306,8 +1306,9 @@ EngineCUDA::FlushPlan EngineCUDA::build_plan(const vector<LoopB> &kernels, const
             if (kernels[k].isSystemOnly()) continue;
             lowered[k] = lower_kernel(kernels[k], cg_opt);
         }
-        // Small dependent order-free reductions run in the tail of the kernel before them. Not
-        // while recording per-kernel timings, whose features describe one kernel each.
+        // Row-wise neighbours run as one kernel and small dependent order-free reductions in the tail
+        // of the kernel before them. Not while recording per-kernel timings, whose features describe
+        // one kernel each (set_record() drops the plans of the other kind).
         if (!record) folded_into = fuse_tails(kernels, lowered, cg_opt);
         for (size_t k = 0; k < kernels.size(); ++k)
             for (const LaunchUnit &u : lowered[k]) all.push_back(&u);
@@ -1386,10 +1387,7 @@ EngineCUDA::FlushPlan EngineCUDA::build_plan(const vector<LoopB> &kernels, const
             }
         }
         pk.writes.assign(writes.begin(), writes.end());
-        // Features of every kernel, whether recording is on or not: a plan built before recording
-        // is switched on is reused by the recorded executions (computing them only when recording
-        // left those kernels with all-zero features).
-        if (!pk.units.empty()) pk.feat = jitk::block_features(kernel);
+        if (record && !pk.units.empty()) pk.feat = jitk::block_features(kernel);
         // Summation order of the floating-point sums and products: "seq" (one thread folds in
         // index order) unless a unit reduces the sweep across threads.
         for (const LoopB *part : parts)

@@ -161,6 +161,9 @@ public:
     bool has_costmodel() const { return cm != nullptr; }
     // Replace the pre-fuser and transformer list (comma-separated names) and forget every plan.
     void set_fusion(const std::string &pre_fuser, const std::string &fuser_list);
+    // Switches recording. Plans are built again: one for recording keeps every kernel apart (a
+    // recorded row describes one), any other fuses small and row-wise kernels.
+    void set_record(bool on);
     // Write the recorded rows (float32: features then microseconds); returns the row count.
     size_t dump_records(const std::string &path) const;
     void clear_records() { records.clear(); }

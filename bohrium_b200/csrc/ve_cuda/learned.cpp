@@ -8,6 +8,8 @@
 //   merge among the legal ones (mergeable(), the plain rule). Every candidate (a, b) is scored by
 //   the predicted gain t(a) + t(b) - t(a merged with b), all predictions of one step computed in
 //   one batched inference on the GPU; the best positive gain is merged, none stops the fuser.
+//   The gain is a ranking: the predictions are of kernels on their own, while tails and row groups
+//   (fuse_tails) are formed after the merges, in either plan.
 // - Keeping a plan: a learned plan is tried only when its floating-point sums and products fold
 //   in the same order as in the greedy plan (so every output is bit-identical to the greedy
 //   form); both plans are timed on the device and the faster one stays for the structure.
@@ -110,6 +112,16 @@ void EngineCUDA::set_fusion(const string &pre_fuser, const string &fuser_list) {
     }
     synchronize();
     fuse_cache.clear();
+    replays.clear();
+    plans.clear();
+    trials.clear();
+    decided.clear();
+}
+
+void EngineCUDA::set_record(bool on) {
+    if (on == record) return;
+    record = on;
+    synchronize();
     replays.clear();
     plans.clear();
     trials.clear();

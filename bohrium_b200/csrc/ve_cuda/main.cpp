@@ -83,7 +83,7 @@ public:
         } else if (msg.rfind("CUDA: prof ", 0) == 0) {
             engine.prof = msg.substr(11) == "on";
         } else if (msg.rfind("CUDA: record ", 0) == 0) {
-            engine.record = msg.substr(13) == "on";
+            engine.set_record(msg.substr(13) == "on");
         } else if (msg.rfind("CUDA: records dump ", 0) == 0) {
             ss << engine.dump_records(msg.substr(19));
             return ss.str();

@@ -5409,9 +5409,12 @@ RowFit lower_rows(const vector<RowStage> &stages, const set<const bh_base *> &un
             else if (!seen.count(x.v->base)) return RowFit::NEVER;
         }
     }
-    // What one stage alone touches is read and written in memory; the others live in registers from
-    // their first stage to their last. Lanes per row: LANE_REDUCE's, more where a row's part of them
+    // What several stages touch lives in registers from the first to the last of them, what one stage
+    // alone writes goes to memory. Lanes per row: LANE_REDUCE's, more where a row's part of them
     // does not fit a lane's registers.
+    vector<RowArray> read_once;  // what one stage alone reads
+    for (const RowArray &r : rows)
+        if (r.first == r.last && r.load && !dropped.count(r.view.base)) read_once.push_back(r);
     rows.erase(remove_if(rows.begin(), rows.end(), [&](const RowArray &r) { return r.first == r.last && !dropped.count(r.view.base); }),
                rows.end());
     int live = 0;
@@ -5432,6 +5435,14 @@ RowFit lower_rows(const vector<RowStage> &stages, const set<const bh_base *> &un
     if (live == 0 || none_of(st.begin(), st.end(), [](const RowStage &x) { return x.reduce; })) return RowFit::NOT_YET;
     if (out == nullptr) return RowFit::FITS;
     LaunchUnit &u = *out;
+    // What one stage reads is loaded before its elements are computed too, as far as registers go: read
+    // where it is used, each load waits for the branches of the element before.
+    for (const RowArray &r : read_once) {
+        int64_t words = (bh_type_size(r.view.base->dtype()) + 3) / 4;
+        for (const RowArray &o : rows)
+            if (o.first <= r.first && r.first <= o.last) words += (bh_type_size(o.view.base->dtype()) + 3) / 4;
+        if (NU * words <= kRowRegisters) rows.push_back(r);
+    }
     for (const bh_base *b : dropped) sym.temps.insert(b);
     // Rebuild the parameters without the dropped arrays.
     {

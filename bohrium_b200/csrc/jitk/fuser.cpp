@@ -529,6 +529,23 @@ vector<InstrPtr> swap_axis(const vector<InstrPtr> &instr_list, int64_t axis1, in
     return ret;
 }
 
+// Free `base` in the loop that holds its last access in `loop`, as the fuser's own blocks do.
+bool free_at_last_access(LoopB &loop, bh_base *base) {
+    for (size_t i = loop._block_list.size(); i-- > 0;) {
+        Block &b = loop._block_list[i];
+        if (b.isInstr()) {
+            for (const bh_view &v : b.getInstr()->getViews())
+                if (v.base == base) {
+                    loop._frees.insert(base);
+                    return true;
+                }
+        } else if (free_at_last_access(b.getLoop(), base)) {
+            return true;
+        }
+    }
+    return false;
+}
+
 vector<Block> swap_blocks(const LoopB &parent, const LoopB *child) {
     vector<Block> ret;
     for (const Block &b : parent._block_list) {
@@ -539,10 +556,13 @@ vector<Block> swap_blocks(const LoopB &parent, const LoopB *child) {
             loop._block_list.push_back(b);
             loop._frees.insert(parent._frees.begin(), parent._frees.end());
         } else {
+            // The child's nest is built anew: its frees, at every depth, and the parent's
             loop.size = child->size;
             const vector<InstrPtr> t = swap_axis(all_instr(*child), parent.rank, child->rank);
             loop._block_list.push_back(create_nested_block(t, child->rank, parent.size));
-            loop._frees.insert(child->_frees.begin(), child->_frees.end());
+            set<bh_base *> frees = child->getAllFrees();
+            frees.insert(parent._frees.begin(), parent._frees.end());
+            for (bh_base *f : frees) free_at_last_access(loop, f);
         }
         loop.metadataUpdate();
         ret.emplace_back(std::move(loop));
@@ -630,7 +650,7 @@ void settle_frees(vector<Block> &block_list, LoopB *parent = nullptr) {
             forget_free(block_list[i].getLoop(), b);
             if (!block_list[it->second].isInstr()) {
                 LoopB &l = block_list[it->second].getLoop();
-                if (!l.getAllFrees().count(b)) l._frees.insert(b);
+                if (!l.getAllFrees().count(b)) free_at_last_access(l, b);
             } else if (parent != nullptr) {
                 parent->_frees.insert(b);
             }

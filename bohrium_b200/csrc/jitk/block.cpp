@@ -405,6 +405,13 @@ vector<const LoopB *> get_first_loop_blocks(const LoopB &block) {
     return ret;
 }
 
+// An accumulate reads the element it wrote before (and starts from one that is set before the loop):
+// nothing else in its loop may write its output.
+bool accumulate_overwritten(const bh_instruction &a, const bh_instruction &b) {
+    return (bh_opcode_is_accumulate(a.opcode) || bh_opcode_is_accumulate(b.opcode)) && !a.operand.empty() && !b.operand.empty() &&
+           !a.operand[0].isConstant() && !b.operand[0].isConstant() && a.operand[0].base == b.operand[0].base;
+}
+
 namespace {
 // Can `writer` and `reader` of the same base run element-wise in one loop nest?
 bool dp_compatible(const bh_view &writer, const bh_view &reader) {
@@ -416,6 +423,7 @@ bool dp_compatible(const bh_view &writer, const bh_view &reader) {
 
 bool dp_compatible(const InstrPtr &a, const InstrPtr &b) {
     if (bh_opcode_is_system(a->opcode) || bh_opcode_is_system(b->opcode)) return true;
+    if (accumulate_overwritten(*a, *b)) return false;
     if (b->opcode == BH_GATHER && a->operand[0].base == b->operand[1].base) return false;
     if (a->opcode == BH_SCATTER || a->opcode == BH_COND_SCATTER) {
         for (const bh_view &v : b->operand)

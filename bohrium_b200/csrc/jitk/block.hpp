@@ -103,6 +103,7 @@ std::vector<const bh_base *> instr_bases(const bh_instruction &instr);
 
 LoopB merge(const LoopB &a, const LoopB &b);
 // Nest `instr_list` from `rank` down to the innermost loop (all instructions share one shape).
+bool accumulate_overwritten(const bh_instruction &a, const bh_instruction &b);
 Block create_nested_block(const std::vector<InstrPtr> &instr_list, int rank = 0, std::set<bh_base *> frees = {});
 // Nest `instr_list` at `rank` with the given loop size (reshaping reshapable instructions).
 Block create_nested_block(const std::vector<InstrPtr> &instr_list, int rank, int64_t size_of_rank_dim);

@@ -62,6 +62,7 @@ bool fully_dp_compatible(const bh_view &writer, const bh_view &reader) {
 
 bool fully_dp_compatible(const InstrPtr &a, const InstrPtr &b) {
     if (bh_opcode_is_system(a->opcode) || bh_opcode_is_system(b->opcode)) return true;
+    if (accumulate_overwritten(*a, *b)) return false;
     if (b->opcode == BH_GATHER && a->operand[0].base == b->operand[1].base) return false;
     if (a->opcode == BH_SCATTER || a->opcode == BH_COND_SCATTER) {
         for (const bh_view &v : b->operand)

@@ -758,6 +758,14 @@ bh_instruction make_identity(const InstrPtr &sweep, int64_t &origin_count) {
     return identity;
 }
 
+// The metadata of a loop and of those in it: the swept instruction, which no longer creates its output,
+// may be in any of them.
+void update_nest(LoopB &loop) {
+    for (Block &b : loop._block_list)
+        if (!b.isInstr()) update_nest(b.getLoop());
+    loop.metadataUpdate();
+}
+
 // Insert identity instructions in front of every swept sub-block (core/jitk/apply_fusion.cpp:87-129).
 void add_identity_block(LoopB &loop, int64_t &origin_count) {
     vector<Block> ret;
@@ -779,7 +787,7 @@ void add_identity_block(LoopB &loop, int64_t &origin_count) {
             bh_instruction updated{*sweep};
             updated.constructor = false;
             block.getLoop().replaceInstr(sweep, updated);
-            block.getLoop().metadataUpdate();
+            update_nest(block.getLoop());
         }
         ret.push_back(block);
     }
@@ -802,7 +810,7 @@ vector<LoopB> add_identity_block(vector<Block> &block_list, int64_t &origin_coun
             bh_instruction updated{*sweep};
             updated.constructor = false;
             block.getLoop().replaceInstr(sweep, updated);
-            block.getLoop().metadataUpdate();
+            update_nest(block.getLoop());
         }
         kernel._block_list.push_back(block);
         kernel.metadataUpdate();

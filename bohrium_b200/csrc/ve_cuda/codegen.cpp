@@ -3810,40 +3810,58 @@ bool scan1d_applicable(const LoopB &loop, InstrPtr &acc) {
     return true;
 }
 
-// The instructions of a SCAN1D loop before its accumulate run once per unit: they may not update an
-// array in place. When some do and no temporary leaves them, `maps` receives the loop of those
-// instructions and `rest` the loop without them (two kernels in order); false when neither holds.
-bool split_in_place_updates(const LoopB &loop, const InstrPtr &acc, LoopB &maps, LoopB &rest, bool &split) {
-    set<const bh_base *> read, written, temps;
-    for (const bh_base *b : loop.getLocalTemps()) temps.insert(b);
-    split = false;
-    bool before = true, crosses = false;
+// The instructions of a SCAN1D loop before its accumulate run once per unit: they may not change what
+// a later unit reads again (an array updated in place, or overwritten after it was read). When some do,
+// `maps` receives a loop of the instructions up to the last such one and `rest` the loop without them:
+// two kernels in order. An instruction that those up to the last update do not need, and whose inputs
+// they leave alone, stays with the scan, which computes it as a register. A temporary that the scan
+// reads but the map has to compute (from values before the update) is an array in memory between them.
+// True when the loop was split.
+bool split_in_place_updates(const LoopB &loop, const InstrPtr &acc, LoopB &maps, LoopB &rest) {
+    vector<InstrPtr> before;
+    set<const bh_base *> read, written;
+    size_t end = 0;  // after the last update
+    for (const Block &b : loop._block_list) {
+        const InstrPtr &i = b.getInstr();
+        if (i == acc) break;
+        if (bh_opcode_is_system(i->opcode)) continue;
+        for (size_t o = 1; o < i->operand.size(); ++o)
+            if (!i->operand[o].isConstant() && !written.count(i->operand[o].base)) read.insert(i->operand[o].base);
+        written.insert(i->operand[0].base);
+        before.push_back(i);
+        if (read.count(i->operand[0].base)) end = before.size();
+    }
+    if (end == 0) return false;
+    // Backwards from the last update: what the map keeps, and what those instructions read and write.
+    set<const bh_instruction *> mapped;
+    set<const bh_base *> reads, writes;
+    for (size_t k = end; k-- > 0;) {
+        const bh_instruction &i = *before[k];
+        const bh_base *out = i.operand[0].base;
+        bool later = k + 1 < end && !reads.count(out) && !writes.count(out) && !read.count(out);
+        for (size_t o = 1; o < i.operand.size(); ++o)
+            if (!i.operand[o].isConstant() && writes.count(i.operand[o].base)) later = false;
+        if (later) continue;
+        mapped.insert(&i);
+        writes.insert(out);
+        for (size_t o = 1; o < i.operand.size(); ++o)
+            if (!i.operand[o].isConstant()) reads.insert(i.operand[o].base);
+    }
     maps = loop;
     rest = loop;
     maps._block_list.clear();
     rest._block_list.clear();
+    set<const bh_base *> in_rest;
     for (const Block &b : loop._block_list) {
         const InstrPtr &i = b.getInstr();
-        if (i == acc) before = false;
-        if (bh_opcode_is_system(i->opcode)) {
-            rest._block_list.push_back(b);
-            continue;
-        }
-        if (before) {
-            for (size_t o = 1; o < i->operand.size(); ++o)
-                if (!i->operand[o].isConstant() && !written.count(i->operand[o].base)) read.insert(i->operand[o].base);
-            written.insert(i->operand[0].base);
-            if (read.count(i->operand[0].base)) split = true;
-            maps._block_list.push_back(b);
-        } else {
-            for (size_t o = 1; o < i->operand.size(); ++o)
-                if (!i->operand[o].isConstant() && temps.count(i->operand[o].base) && written.count(i->operand[o].base))
-                    crosses = true;
-            rest._block_list.push_back(b);
-        }
+        (mapped.count(i.get()) ? maps : rest)._block_list.push_back(b);
+        if (bh_opcode_is_system(i->opcode) || mapped.count(i.get())) continue;
+        for (const bh_view &v : i->operand)
+            if (!v.isConstant()) in_rest.insert(v.base);
     }
-    if (!split) return true;
-    if (crosses) return false;
+    // Arrays are freed by the last loop that accesses them; one that the map creates and the rest
+    // frees is no temporary of either.
+    for (bh_base *b : loop._frees) (in_rest.count(b) || !(reads.count(b) || writes.count(b)) ? maps : rest)._frees.erase(b);
     maps.metadataUpdate();
     rest.metadataUpdate();
     return true;
@@ -5934,13 +5952,12 @@ vector<LaunchUnit> lower_kernel(const LoopB &kernel, const CodegenOptions &opt) 
                 const bh_view &v = jitk::all_instr(*il)[0]->operand[0];
                 ok = ok && v.base == scan_acc->operand[0].base;
             }
-            LoopB maps, rest;
-            bool split = false;
-            ok = ok && split_in_place_updates(L, scan_acc, maps, rest, split);
             if (ok) {
                 pending_id_loops.clear();
-                if (split) units.push_back(lower_flat(maps, 1, opt));
-                const LoopB &S = split ? rest : L;
+                LoopB S = L;
+                // (the rest may update what a map before it wrote)
+                for (LoopB maps, rest; split_in_place_updates(S, scan_acc, maps, rest); S = rest)
+                    units.push_back(lower_flat(maps, 1, opt));
                 if (opt.scan_single_pass && !opt.bounds_check) {
                     units.push_back(lower_scan1d_single(S, scan_acc, opt));
                 } else {

@@ -140,12 +140,13 @@ def test_values(gpu_rt, prog, dtype, n):
 @pytest.mark.gpu
 @pytest.mark.parametrize("batch", ["off", "grouped", "graph"])
 def test_repeated_flushes(gpu_executor, batch):
-    """The plan's replays update the array once more each time."""
+    """The plan's replays update the array once more each time. The values grow with every replay, past
+    what float64 holds exactly: 64-bit integers, whose sums are exact modulo 2^64 in any order."""
     gpu_executor.message("CUDA: batch " + batch)
     try:
         rt = bh.Runtime(gpu_executor)
         rng = np.random.default_rng(4)
-        x, y = rng.integers(-3, 4, 50_001).astype(np.float64), rng.integers(-3, 4, 50_001).astype(np.float64)
+        x, y = rng.integers(-3, 4, 50_001), rng.integers(-3, 4, 50_001)
         for prog in PROGRAMS:
             a, b = bh.array(rt, x), bh.array(rt, y)
             rt.flush()

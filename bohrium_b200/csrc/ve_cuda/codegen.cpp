@@ -1483,14 +1483,6 @@ void emit_preload(Emitter &em, const vector<bh_view> &views, int V, const string
     for (size_t k = 0; k < views.size(); ++k) scope.repl[ViewKey(views[k])] = "pl" + to_string(k) + "[j]";
 }
 
-// 128-bit access for FLAT: thread t of a work item handles the 4 consecutive elements
-// cbase .. cbase + 3 (cbase = chunk * 1024 + 4t) of the innermost parallel rank, so a view with
-// unit stride along it is one 16-byte (or 4 x element size) word per thread. Read-only such views
-// are loaded, and arrays written by the element code stored, as whole words when every such view's
-// first element is aligned to the word (checked per work item); otherwise, and for views with other
-// strides, element by element. The written values stay in registers until the words are stored,
-// and later reads of them in the element code use the registers. Every element is computed by the
-// same statements either way, so the results do not depend on the path.
 // True when the instructions of `L` read view `v`'s array before they write it: an update in place,
 // whose register copy has to start from the array's value.
 bool read_before_written(const LoopB &L, const bh_view &v) {
@@ -1614,6 +1606,14 @@ void emit_flat_strided(Symbols &sym, ostream &body, const CodegenOptions &opt, c
     body << "        }\n    }\n";
 }
 
+// 128-bit access for FLAT: thread t of a work item handles the 4 consecutive elements
+// cbase .. cbase + 3 (cbase = chunk * 1024 + 4t) of the innermost parallel rank, so a view with
+// unit stride along it is one 16-byte (or 4 x element size) word per thread. Read-only such views
+// are loaded, and arrays written by the element code stored, as whole words when every such view's
+// first element is aligned to the word (checked per work item); otherwise, and for views with other
+// strides, element by element. The written values stay in registers until the words are stored,
+// and later reads of them in the element code use the registers. Every element is computed by the
+// same statements either way, so the results do not depend on the path.
 void emit_flat_vector(Symbols &sym, ostream &body, const CodegenOptions &opt, const LoopB &inner,
                       const vector<const LoopB *> &chain, unsigned P, const vector<bh_view> &pre, int64_t per,
                       const FlatIndex &fi) {
@@ -1873,7 +1873,8 @@ LaunchUnit lower_flat(const LoopB &loop, unsigned P, const CodegenOptions &opt) 
 // shared-memory ring by one TMA copy per tile, up to 2 tiles ahead, with the 128-byte swizzle; a
 // thread reads its TR/4 values as two 16-byte words (distinct banks across every 8 threads).
 constexpr int kTileCols = 64;
-// Two stages: 32 KB for two views, so six CTAs fit on an SM. Four stages and three CTAs hold the
+// Two stages: 33 KB of ring for two views and 8.3 KB of boxes for the path without TMA, so five CTAs fit on an
+// SM (48 registers a thread; four with two transposed views). Four stages and three CTAs hold the
 // same bytes in flight with half the warps to store them (float32 8192 x 6000 on a B200: 115 and
 // 108 us, 2048 x 2048 13.9 and 11.9 us, 8192 x 8192 148 and 144 us).
 constexpr int kTileStages = 2;
@@ -2169,9 +2170,9 @@ bool lower_tile2d(const LoopB &loop, const CodegenOptions &opt, LaunchUnit &u) {
     return true;
 }
 
-// Parallel points below which an inner reduction is split along its swept axis, and the number of
-// (point, chunk) threads the split aims at. Both are fixed constants so that the summation order
-// depends on the array shapes only.
+// A reduction along an axis is split where its points alone are fewer than kSplitTargetThreads and the
+// axis holds at least two chunks of kSplitMinChunk (split_chunks() > 1); how it is split is
+// split_shape()'s matter. Fixed constants, so that the summation order depends on the array shapes only.
 constexpr int64_t kSplitTargetThreads = 600000;
 constexpr int64_t kSplitMinChunk = 16;
 // Points from which LANE_REDUCE (C lanes of one CTA per point) fills the GPU well enough to be

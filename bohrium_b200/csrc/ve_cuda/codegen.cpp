@@ -3868,6 +3868,22 @@ bool split_in_place_updates(const LoopB &loop, const InstrPtr &acc, LoopB &maps,
     return true;
 }
 
+// Whether instructions after the accumulate write an array that it or those before it read. The single
+// pass's fallback starts the whole scan again and would read it changed.
+bool inputs_change_after_scan(const LoopB &loop, const InstrPtr &acc) {
+    set<const bh_base *> read;
+    bool after = false;
+    for (const Block &b : loop._block_list) {
+        const InstrPtr &i = b.getInstr();
+        if (bh_opcode_is_system(i->opcode) || i->operand.empty()) continue;
+        if (after && read.count(i->operand[0].base)) return true;
+        for (size_t o = 1; !after && o < i->operand.size(); ++o)
+            if (!i->operand[o].isConstant()) read.insert(i->operand[o].base);
+        after = after || i == acc;
+    }
+    return false;
+}
+
 vector<LaunchUnit> lower_scan1d(const LoopB &loop, const InstrPtr &acc, const CodegenOptions &opt) {
     const Block holder(loop);
     const LoopB &L = holder.getLoop();
@@ -5959,7 +5975,7 @@ vector<LaunchUnit> lower_kernel(const LoopB &kernel, const CodegenOptions &opt) 
                 // (the rest may update what a map before it wrote)
                 for (LoopB maps, rest; split_in_place_updates(S, scan_acc, maps, rest); S = rest)
                     units.push_back(lower_flat(maps, 1, opt));
-                if (opt.scan_single_pass && !opt.bounds_check) {
+                if (opt.scan_single_pass && !opt.bounds_check && !inputs_change_after_scan(S, scan_acc)) {
                     units.push_back(lower_scan1d_single(S, scan_acc, opt));
                 } else {
                     for (LaunchUnit &su : lower_scan1d(S, scan_acc, opt)) units.push_back(std::move(su));

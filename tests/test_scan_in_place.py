@@ -121,6 +121,16 @@ def test_a_map_that_the_scan_can_compute_stays_with_it():
     assert [u["bytes"] for u in got[1:]] == [u["bytes"] for u in alone]
 
 
+def test_the_single_pass_does_not_take_scans_whose_inputs_change(monkeypatch):
+    """Its fallback would read the changed input: the update after the accumulate keeps the three units."""
+    monkeypatch.setenv("BH_CUDA_SCAN_SINGLE_PASS", "true")
+    for prog, want in [(scan_of_the_old_values, 3), (scan_of_a_map, 1)]:
+        rt = bh.Runtime(bh.DryRunExecutor())
+        keep = prog(bh.empty(rt, (3_000_000,), np.float64), None)
+        scheds = [u["sched"] for k in bh.dry_run(rt.take(), compile=True)["kernels"] for u in k["units"]]
+        assert scheds.count("scan1d") == want and len(keep)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("n", [1000, 2048, 50_001, 3_000_017])
 @pytest.mark.parametrize("dtype", [np.float64, np.int32])
@@ -162,3 +172,24 @@ def test_repeated_flushes(gpu_executor, batch):
             rt.flush()
     finally:
         gpu_executor.message("CUDA: batch off")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prog", [scan_of_the_old_values, overwritten_after_it_was_read, scan_of_a_map], ids=lambda f: f.__name__)
+def test_single_pass_that_gives_up(monkeypatch, prog):
+    """The single-pass scan with a negative wait cap redoes what the update may have changed."""
+    for key, value in [("SCAN_SINGLE_PASS", "true"), ("SCAN_SPIN_CAP", "-1"), ("CACHE_DIR", "NONE")]:
+        monkeypatch.setenv("BH_CUDA_" + key, value)
+    ex = bh.NativeExecutor(stack="cuda")
+    try:
+        rng = np.random.default_rng(5)
+        x, y = rng.integers(-3, 4, 300_001), rng.integers(-3, 4, 300_001)
+        rt = bh.Runtime(ex)
+        a, b = bh.array(rt, x), bh.array(rt, y)
+        rt.flush()
+        got = prog(a, b)
+        rt.flush()
+        for g, w in zip(got, prog(x, y)):
+            np.testing.assert_array_equal(g.numpy(), w)
+    finally:
+        ex.close()

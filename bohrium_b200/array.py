@@ -239,15 +239,13 @@ class BhArray:
 
 
 # ------------------------------------------------------------------------------ construction
-_INT = {int}
-
-
 def empty(rt: Runtime, shape, dtype=np.float64) -> BhArray:
-    shape = (shape,) if isinstance(shape, numbers.Integral) else tuple(shape)
-    if not _INT.issuperset(map(type, shape)):  # NumPy integers: their product wraps in their type
-        shape = tuple(map(int, shape))
-    base = rt.new_base(dtype, math.prod(shape))
-    return BhArray(rt, base, 0, shape, _contig_strides(shape))
+    # Python integers: a product of NumPy's would wrap in their type
+    shape = (int(shape),) if isinstance(shape, numbers.Integral) else tuple(map(int, shape))
+    a = BhArray.__new__(BhArray)  # (what __init__ would convert is converted)
+    a.rt, a.base, a.start = rt, rt.new_base(dtype, math.prod(shape)), 0
+    a.shape, a.strides, a._owner = shape, _contig_strides(shape), None
+    return a
 
 
 def full(rt: Runtime, shape, value, dtype=np.float64) -> BhArray:

@@ -3978,7 +3978,7 @@ vector<LaunchUnit> lower_scan1d(const LoopB &loop, const InstrPtr &acc, const Co
         body << block_scan_fn(T, "bh_block_scan", rop, ident);
         // The streaming units' code for full chunks has no bounds checks (64-bit comparisons for every
         // element of every step): with the warp offsets of the block scan folded by every thread
-        // instead of one, 257 -> 239 us for 5e7 float64 (82 + 15 + 151 launch by launch; 62 and 124 for
+        // instead of one, 257 -> 239 us for 5e7 float64 on one GPU and 245 -> 235 on another (82 + 15 + 151 launch by launch; 62 and 124 for
         // the streaming units' bytes at the measured copy rate).
         if (pf) body << "// bh_dynamic_shared_bytes: " << pf_bytes << "\n";
         if (phase == 1) {

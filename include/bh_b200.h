@@ -178,9 +178,9 @@ int bh_ve_cuda_costmodel_train(bh_costmodel *cm, const float *x, const float *t,
  * with its tile partials in a fixed static device array (65,792 bytes per device) instead of
  * allocated scratch, for callers that cannot let a library allocate device memory. It calls no
  * cudaMalloc, cudaFree or other allocating routine. n is at most 16,777,216 (8,192 tiles of 2,048);
- * larger n is rejected with an error. The first call on each device, made with that device
- * current, does a one-time set-up (cudaGetSymbolAddress of the array); make it before any stream
- * capture. All calls share the array: calls whose kernels overlap on the GPU race. Returns 0, or
+ * larger n is rejected with an error. An engine created on a device does its one-time set-up
+ * there; without one the first call on the device, made with it current, looks the array up
+ * (cudaGetSymbolAddress): make that before any stream capture. All calls share the array: calls whose kernels overlap on the GPU race. Returns 0, or
  * -1 with bhb_last_error() set. */
 int bh_ve_cuda_sum_f64_noalloc(const double *in, int64_t n, double *out, void *stream);
 

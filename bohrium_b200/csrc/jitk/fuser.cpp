@@ -872,8 +872,12 @@ vector<LoopB> get_kernel_list(const vector<bh_instruction *> &instr_list, const 
     vector<LoopB> ret;
     if (config.avoid_rank0_sweep) {
         for (Block &b : block_list) {
-            if (b.isInstr() || !b.getLoop()._sweeps.empty()) {
+            if (b.isInstr()) {
                 ret.emplace_back(LoopB{-1, 1, {std::move(b)}});
+            } else if (!b.getLoop()._sweeps.empty()) {
+                // (the reference hands these to a CPU engine, which sets their outputs first itself)
+                vector<Block> one{std::move(b)};
+                for (LoopB &kernel : add_identity_block(one, origin_count)) ret.emplace_back(std::move(kernel));
             } else {
                 LoopB kernel{-1, 1, {std::move(b)}};
                 add_identity_block(kernel, origin_count);

@@ -48,3 +48,39 @@ def test_values_of_an_updated_accumulate(gpu_rt, prog, shape):
     gpu_rt.flush()
     for g, w in zip(got, prog(x)):
         np.testing.assert_array_equal(g.numpy(), w)
+
+
+def accumulate_of_an_accumulate(x):
+    c = accumulated(x, 0)
+    return [accumulated(c, 0) + x, c]
+
+
+def test_sweeps_apart_from_maps_are_seeded_too(monkeypatch):
+    """With avoid_rank0_sweep the sweeping loops are kernels of their own: the accumulates of a loop that
+    no schedule takes start from the identity that an instruction before the loop writes."""
+    monkeypatch.setenv("BH_CUDA_AVOID_RANK0_SWEEP", "true")
+    rt = bh.Runtime(bh.DryRunExecutor())
+    keep = accumulate_of_an_accumulate(bh.empty(rt, (5000,), np.int64))
+    blocks = [k["block"] for k in bh.dry_run(rt.take(), compile=True)["kernels"]]
+    outs = re.findall(r"BH_ADD_ACCUMULATE (a\d+)\[", "".join(b.split("block list:", 1)[1] for b in blocks))
+    assert len(keep) and len(set(outs)) == 2
+    for out in set(outs):
+        assert any(re.search(rf"BH_IDENTITY {out}\[0:1:1\] 0\n", b) for b in blocks)
+
+
+@pytest.mark.gpu
+def test_values_of_sweeps_apart_from_maps(monkeypatch):
+    monkeypatch.setenv("BH_CUDA_AVOID_RANK0_SWEEP", "true")
+    ex = bh.NativeExecutor(stack="cuda")
+    try:
+        rt = bh.Runtime(ex)
+        for seed in range(5):
+            x = values((5000,), np.int64, seed)
+            a = bh.array(rt, x)
+            rt.flush()
+            got = accumulate_of_an_accumulate(a)
+            rt.flush()
+            for g, w in zip(got, accumulate_of_an_accumulate(x)):
+                np.testing.assert_array_equal(g.numpy(), w)
+    finally:
+        ex.close()

@@ -753,8 +753,12 @@ bh_instruction make_identity(const InstrPtr &sweep, int64_t &origin_count) {
     identity.constant = sweep_identity(sweep->opcode, sweep->operand[0].base->dtype());
     identity.origin_id = origin_count++;
     identity.constructor = sweep->constructor;
-    // Accumulates run serially along the swept axis: only its first element is the identity.
-    if (bh_opcode_is_accumulate(sweep->opcode)) identity.operand[0].shape[sweep->sweep_axis()] = 1;
+    // Accumulates run serially along the swept axis: only its first element is the identity (an empty
+    // axis has none: its array has no memory to write).
+    if (bh_opcode_is_accumulate(sweep->opcode)) {
+        int64_t &n = identity.operand[0].shape[sweep->sweep_axis()];
+        n = min<int64_t>(n, 1);
+    }
     return identity;
 }
 

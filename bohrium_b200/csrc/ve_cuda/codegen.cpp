@@ -5983,7 +5983,7 @@ vector<LaunchUnit> lower_kernel(const LoopB &kernel, const CodegenOptions &opt) 
                 continue;
             }
         }
-        bool all_reduce = !L._sweeps.empty();
+        bool all_reduce = !L._sweeps.empty() && L.size > 0;  // (of nothing: the identities, written in order)
         for (const InstrPtr &s : L._sweeps) all_reduce = all_reduce && bh_opcode_is_reduction(s->opcode);
         if (all_reduce && L.isInnermost() && pending_id_loops.empty()) {
             // Every folded identity must belong to one of this loop's reductions.

@@ -5267,6 +5267,7 @@ constexpr int kRowRegisters = 48;        // 4-byte registers of a row that a lan
 // float32 20000 x 1500 (6 words) 250 -> 120, 455 -> 235, 865 -> 749; two softmaxes of one matrix (5 stages, 11
 // instructions) 334 -> 269 at 24 words, four (9, 21) 662 -> 904 there, 861 -> 602 at 12 and 488 -> 216 at 6;
 // 20 instructions in 5 stages 377 -> 594 at 24 words, 493 -> 484 at 12 and 273 -> 172 at 6.
+// Cut at the bound the chains of 16 take 1383 us at 24 words, 1057 at 12 and 470 at 6.
 constexpr int64_t kRowCost = 33000;
 // Stages of a group, where rows are short: 17 in one unit took 181 us and in units of 6 and of 8 113 and 120
 // us (float32 20000 x 300), 9 in one unit 51 us and in units of 6 and 3 58 us.
